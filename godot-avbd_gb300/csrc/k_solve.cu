@@ -36,10 +36,10 @@ struct Blk {
 // Block::Block (types.hpp:157-172).
 __device__ __forceinline__ Blk makeBlock(real mass, f3 moment, real dtSq, f3 x, f3 xi, q4 q, q4 qi) {
     Blk b;
-    const f3 mo = divs(f3{mass, mass, mass}, dtSq);
-    b.lin = mdiag(mo.x, mo.y, mo.z);
+    const real mo = mass / dtSq;
+    b.lin = mdiag(mo, mo, mo);
     b.crs = mzero();
-    b.rl = cmul(mo, sub(x, xi));
+    b.rl = scale(sub(x, xi), mo);
     const m3 rot = qmat(q);
     const m3 iw = mul(rot, mul(mdiag(moment.x, moment.y, moment.z), transpose(rot)));
     b.ang = mdivs(iw, dtSq);
@@ -49,9 +49,13 @@ __device__ __forceinline__ Blk makeBlock(real mass, f3 moment, real dtSq, f3 x, 
 
 // ---- 6x6 solves (maths.h:156-343) ----
 
-__device__ bool ldlt6(const real a[6][6], const real b[6], real x[6]) {
+// QUOTIENTS: a column's quotients by its pivot are found together (dmath.cuh), and so are the final
+// ones; `ok` is cleared where an operand is outside their range, and x is then not to be used.
+template <bool QUOTIENTS>
+__device__ __forceinline__ bool ldlt6Run(const real a[6][6], const real b[6], real x[6], bool &ok) {
     real l[6][6];
     real dd[6];
+    Divisor dv[6];
 #pragma unroll
     for (int j = 0; j < 6; j++) {
         real dj = a[j][j];
@@ -61,6 +65,8 @@ __device__ bool ldlt6(const real a[6][6], const real b[6], real x[6]) {
         if (!(dj > 1.0e-12f))
             return false;
         dd[j] = dj;
+        if (QUOTIENTS)
+            dv[j] = divisor(dj, ok);
         l[j][j] = 1.0f;
 #pragma unroll
         for (int i = j + 1; i < 6; i++) {
@@ -68,7 +74,7 @@ __device__ bool ldlt6(const real a[6][6], const real b[6], real x[6]) {
 #pragma unroll
             for (int s = 0; s < j; s++)
                 lij -= l[i][s] * l[j][s] * dd[s];
-            l[i][j] = lij / dd[j];
+            l[i][j] = QUOTIENTS ? quotient(lij, dv[j], ok) : lij / dd[j];
         }
     }
     real z[6];
@@ -82,7 +88,7 @@ __device__ bool ldlt6(const real a[6][6], const real b[6], real x[6]) {
     }
 #pragma unroll
     for (int i = 0; i < 6; i++)
-        x[i] = z[i] / dd[i];
+        x[i] = QUOTIENTS ? quotient(z[i], dv[i], ok) : z[i] / dd[i];
 #pragma unroll
     for (int i = 5; i >= 0; i--) {
         real v = x[i];
@@ -223,34 +229,37 @@ struct Delta {
     bool ok;
 };
 
-// solve()'s pivoted fallback, out of line: the block travels by value, so the fast path's matrix
-// never needs an address and stays in registers.
-__device__ __noinline__ Delta solvePivoted(Blk k) {
+// Block::solveDelta with solve()'s fallback chain (plain LDLT, pivoted LDLT), out of line: the block
+// travels by value, so the fast path's matrix never needs an address and stays in registers.
+__device__ __noinline__ Delta solveSlow(Blk k) {
     real a[6][6], b[6], x[6];
     blockSystem(k, a, b);
+    bool ok = true;
     Delta r;
-    r.ok = ldlt6Pivoted(a, b, x);
+    r.ok = ldlt6Run<false>(a, b, x, ok) || ldlt6Pivoted(a, b, x);
     r.dl = f3{x[0], x[1], x[2]};
     r.da = f3{x[3], x[4], x[5]};
     return r;
 }
 
-// Block::solveDelta's plain LDLT; false when solve() would fall back.
+// The plain LDLT with grouped quotients; false when it fails or an operand is outside their range
+// (solveSlow then gives the result).
 __device__ __forceinline__ bool solveBlockFast(const Blk &k, f3 &dl, f3 &da) {
     real a[6][6], b[6], x[6];
     blockSystem(k, a, b);
-    if (!ldlt6(a, b, x))
+    bool ok = true;
+    if (!ldlt6Run<true>(a, b, x, ok) || !ok)
         return false;
     dl = f3{x[0], x[1], x[2]};
     da = f3{x[3], x[4], x[5]};
     return true;
 }
 
-// Block::solveDelta with solve()'s fallback chain: plain LDLT, pivoted LDLT, then no step.
+// Block::solveDelta: plain LDLT, pivoted LDLT, then no step.
 __device__ __forceinline__ void solveBlock(const Blk &k, f3 &dl, f3 &da) {
     if (solveBlockFast(k, dl, da))
         return;
-    const Delta r = solvePivoted(k);
+    const Delta r = solveSlow(k);
     if (r.ok) {
         dl = r.dl;
         da = r.da;
@@ -976,7 +985,7 @@ __device__ __forceinline__ void applyOverflow(const Dev &d, const StepParams &p,
     }
 }
 
-// solve()'s pivoted fallback for a body whose plain LDLT failed, out of line so the common path
+// solve()'s fallback for a body the fast path left, out of line so the common path
 // keeps its registers; the kernel's parameters are grid constants, so the call passes their
 // addresses without copying them. The block is assembled again (the same floats: it reads the
 // stamps, this body's own pose, which it has not written yet, and for a body with a force its
@@ -985,7 +994,7 @@ template <bool FORCES, bool RO = true>
 __device__ __noinline__ void fallbackSolve(const Dev &d, const StepParams &p, int g, int inPlace) {
     Blk blk = bodyBlock(d, p, g);
     assemble<false, FORCES, RO>(d, p, g, blk);
-    const Delta r = solvePivoted(blk);
+    const Delta r = solveSlow(blk);
     applyOverflow(d, p, g, inPlace, r.ok ? r.dl : f3{0, 0, 0}, r.ok ? r.da : f3{0, 0, 0});
 }
 
