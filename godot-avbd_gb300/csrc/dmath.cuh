@@ -192,6 +192,10 @@ AVBD_HD f3 mul(const m3 &a, f3 b) { return add(add(scale(a.c0, b.x), scale(a.c1,
 AVBD_HD m3 mul(const m3 &a, const m3 &b) { return m3{mul(a, b.c0), mul(a, b.c1), mul(a, b.c2)}; }
 AVBD_HD m3 madd(const m3 &a, const m3 &b) { return m3{add(a.c0, b.c0), add(a.c1, b.c1), add(a.c2, b.c2)}; }
 AVBD_HD m3 mscale(const m3 &a, real s) { return m3{scale(a.c0, s), scale(a.c1, s), scale(a.c2, s)}; }
+AVBD_HD m3 mdivsPlain(const m3 &a, real s) {
+    return m3{f3{a.c0.x / s, a.c0.y / s, a.c0.z / s}, f3{a.c1.x / s, a.c1.y / s, a.c1.z / s},
+              f3{a.c2.x / s, a.c2.y / s, a.c2.z / s}};
+}
 AVBD_HD m3 mdivs(const m3 &a, real s) {
 #if defined(__CUDA_ARCH__) && !defined(AVBDG_FP64)
     bool ok = true;
@@ -202,8 +206,7 @@ AVBD_HD m3 mdivs(const m3 &a, real s) {
     if (ok)
         return q;
 #endif
-    return m3{f3{a.c0.x / s, a.c0.y / s, a.c0.z / s}, f3{a.c1.x / s, a.c1.y / s, a.c1.z / s},
-              f3{a.c2.x / s, a.c2.y / s, a.c2.z / s}};
+    return mdivsPlain(a, s);
 }
 AVBD_HD m3 mneg(const m3 &a) { return m3{neg(a.c0), neg(a.c1), neg(a.c2)}; }
 

@@ -78,7 +78,10 @@ void layoutStore(Dev &n, int nb, int mm, int ff, int pp, int ww, bool arm, Take 
     n.WW = ww;
     take(n.wBase, ww);
     take(n.wCount, ww);
-    take(n.wMaxDepth, ww);
+    take(n.wMan, static_cast<size_t>(ww) + 1);
+    take(n.wOldFirst, static_cast<size_t>(ww) + 1);
+    take(n.wNewFirst, static_cast<size_t>(ww) + 1);
+    take(n.wMaxDepth, 2 * static_cast<size_t>(ww));
     take(n.wStop, ww);
     take(n.wBounds, 6 * static_cast<size_t>(ww));
     take(n.wActive, ww);
@@ -218,6 +221,8 @@ Engine::Engine(const avbdg_params &params, int maxBodies, int maxForces, int max
     roundQueue = queue && queue[0] == '1';
     const char *noBrute = std::getenv("AVBDG_NO_BRUTE");
     bruteAllowed = !(noBrute && noBrute[0] == '1');
+    const char *noWorld = std::getenv("AVBDG_NO_WORLD");
+    worldAllowed = !(noWorld && noWorld[0] == '1') && !roundQueue;
     const char *noTune = std::getenv("AVBDG_NO_TUNE");
     tuneEnabled = !(noTune && noTune[0] == '1');
 #ifdef AVBDG_FP64
@@ -884,14 +889,55 @@ Engine::StepPlan Engine::planStep(int mode, int substeps, int rounds) {
     plan.greedy = needGreedy();
     plan.multiWorld = worlds() > 1;
     plan.round = nRound > 0;
+    int most = 1;
+    for (int c : wCount)
+        most = std::max(most, c);
+    int count = 1; // worlds, rounded up: a plan then serves a range of them
+    while (count < worlds())
+        count *= 2;
+    const int bodies = worlds() > 1 ? (most + 7) / 8 * 8 : most;
+    plan.worldMajor = worldAllowed && worlds() > 1 && nBodies <= kWorldMajorBodies;
+    if (plan.worldMajor != liveByWorld) {
+        if (plan.worldMajor)
+            sortLiveByWorld();
+        liveByWorld = plan.worldMajor || worlds() <= 1; // (a single world's order is its own)
+    }
+    if (worldAllowed && !plan.greedy && (plan.worldMajor || worlds() == 1)) {
+        // Manifolds a body in the last checked step (a store's first step: a settled pile's).
+        const double density = ctrFresh && nBodies > 0 ? static_cast<double>(hostCtr[C_LIVE]) / nBodies : 2.5;
+        if (worldsTake(count, bodies, density)) {
+            plan.worldCount = count;
+            plan.worldBodies = bodies;
+        }
+    }
     return plan;
+}
+
+// The live manifolds in world order, each world's own order kept: from here on each step leaves them so.
+void Engine::sortLiveByWorld() {
+    if (cudaStreamSynchronize(stream) != cudaSuccess)
+        return; // (the step reports it)
+    int live = 0;
+    cudaMemcpy(&live, d.ctr + C_LIVE, sizeof(int), cudaMemcpyDeviceToHost);
+    std::vector<int2> ab(static_cast<size_t>(std::max(live, 0)));
+    if (ab.empty())
+        return;
+    cudaMemcpy(ab.data(), d.live.ab, sizeof(int2) * ab.size(), cudaMemcpyDeviceToHost);
+    std::vector<int> order(ab.size()), places(ab.size());
+    for (size_t i = 0; i < order.size(); i++)
+        order[i] = static_cast<int>(i);
+    const auto world = [&](int m) { return std::upper_bound(wBase.begin(), wBase.end(), ab[m].x) - wBase.begin(); };
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return world(a) < world(b); });
+    for (size_t i = 0; i < order.size(); i++)
+        places[order[i]] = static_cast<int>(i);
+    launchManifoldPermute(d, places, stream); // (the step rebuilds the adjacency's manifold numbers after this)
 }
 
 std::string Engine::StepPlan::key() const {
     char buf[128];
-    std::snprintf(buf, sizeof(buf), "%d/%d/%d/%d%d%d%d%d%d%d%d", mode, substeps, rounds, adjAtStart ? 1 : 0,
+    std::snprintf(buf, sizeof(buf), "%d/%d/%d/%d%d%d%d%d%d%d%d%d/%d/%d", mode, substeps, rounds, adjAtStart ? 1 : 0,
                   anyTree ? 1 : 0, rebuild ? 1 : 0, forces ? 1 : 0, greedy ? 1 : 0, multiWorld ? 1 : 0,
-                  round ? 1 : 0, brute ? 1 : 0);
+                  round ? 1 : 0, brute ? 1 : 0, worldMajor ? 1 : 0, worldCount, worldBodies);
     return buf;
 }
 
@@ -909,6 +955,7 @@ int Engine::broadPhase(const StepParams &sp, const StepPlan &plan) {
     if (!plan.anyTree) {
         cudaMemsetAsync(d.ctr + C_PAIRS, 0, sizeof(int), stream);
         cudaMemcpyAsync(d.ctr + C_CAND, d.ctr + C_LIVE, sizeof(int), cudaMemcpyDeviceToDevice, stream);
+        cudaMemcpyAsync(d.ctr + C_OLDLIVE, d.ctr + C_LIVE, sizeof(int), cudaMemcpyDeviceToDevice, stream);
         return AVBDG_OK;
     }
     // The tree is rebuilt on the reference's schedule either way (its codes and order are dumped);
@@ -939,7 +986,14 @@ bool Engine::enqueueStep(const StepPlan &plan) {
         recordPhase(ev[1]);
         if (!launchesOk())
             return false;
-        warmstartAndSelect(sp);
+        warmstartAndSelect(sp, plan);
+        if (plan.worldCount) {
+            recordPhase(ev[2]);
+            if (launchesOk())
+                runWorlds(sp, plan);
+            recordPhase(ev[3]);
+            return launchesOk();
+        }
         projectContacts(sp, false, 0.0f);
         recordPhase(ev[2]);
         if (!launchesOk())
@@ -958,8 +1012,14 @@ bool Engine::enqueueStep(const StepPlan &plan) {
     recordPhase(ev[1]);
     if (!launchesOk())
         return false;
-    warmstartAndSelect(sp);
+    warmstartAndSelect(sp, plan);
     recordPhase(ev[2]);
+    if (plan.worldCount) {
+        if (launchesOk())
+            runWorlds(sp, plan);
+        recordPhase(ev[3]);
+        return launchesOk();
+    }
     for (int sub = 0; sub < substeps; ++sub) {
         if (!launchesOk())
             return false;
@@ -1084,12 +1144,12 @@ int Engine::runPlan(const StepPlan &plan) {
 }
 
 // warmstartForces + selectUpdateBodies (solver_solve.cpp:31-105, 263-424).
-int Engine::warmstartAndSelect(const StepParams &sp) {
+int Engine::warmstartAndSelect(const StepParams &sp, const StepPlan &plan) {
     launchForceInit(d, sp, nForces > 0, stream);
     beginSpan();
     launchManifoldInit(d, sp, nRound > 0, tuned.narrow, stream);
     endSpan(kNarrow);
-    launchManifoldCompact(d, stream);
+    launchManifoldCompact(d, plan.worldMajor, stream);
     launchAdjacency(d, stream);
     if (sp.sleepFrames > 0)
         launchSleepSelect(d, sp, stream);
@@ -1108,18 +1168,41 @@ void Engine::projectContacts(const StepParams &sp, bool positions, real window) 
         launchProjection(d, sp, stream);
 }
 
+// Rounds of a substep that run the primal.
+int Engine::newtonRoundsOf(int rounds) const {
+    return std::clamp(static_cast<int>(std::ceil(P.newton_ratio * static_cast<float>(rounds))), 1, rounds);
+}
+
+// Convergence probe (solver_step.cpp:88, 301-314): after each round but the last, the mean
+// step-start penetration r (a mean of positive floats, so 0 <= r <= inf) is compared with the
+// previous probe's, starting from 0; the first probe's 0 - r < threshold holds for every
+// threshold > 0, so a positive threshold always stops the substep after its first round.
+int Engine::roundsRun(int rounds) const { return (P.convergence_threshold > 0.0f && rounds > 1) ? 1 : rounds; }
+
+// Everything after the adjacency and the colouring, a cluster per world (the phases of enqueueStep's
+// separate launches, in their order).
+void Engine::runWorlds(const StepParams &sp, const StepPlan &plan) {
+    WorldRun run{};
+    const int rounds = plan.mode == 0 ? P.iterations : plan.rounds;
+    run.substeps = plan.mode == 0 ? 1 : plan.substeps;
+    run.rounds = roundsRun(rounds);
+    run.newtonRounds = newtonRoundsOf(rounds);
+    run.dt = P.dt;
+    run.tolerance = std::max(static_cast<real>(sp.projSlop * 0.01f), static_cast<real>(1.0e-6f));
+    run.brake = sp.specMargin > 0.0f;
+    run.project = P.position_projection != 0 && sp.projIters > 0;
+    run.colours = needGreedy();
+    run.multiWorld = plan.multiWorld;
+    launchWorlds(d, sp, run, plan.worldCount, plan.worldBodies, stream);
+}
+
 // Solver::runSubstep + iterateBody (solver_step.cpp:79-105, 195-316).
 void Engine::runSubstep(const StepParams &sp, int rounds, bool idle) {
     launchWarmstartBodies(d, sp, stream);
-    const int newtonRounds =
-            std::clamp(static_cast<int>(std::ceil(P.newton_ratio * static_cast<float>(rounds))), 1, rounds);
+    const int newtonRounds = newtonRoundsOf(rounds);
     const bool colours = needGreedy();
     const bool inPlace = nForces == 0;
-    // Convergence probe (solver_step.cpp:88, 301-314): after each round but the last, the mean
-    // step-start penetration r (a mean of positive floats, so 0 <= r <= inf) is compared with the
-    // previous probe's, starting from 0; the first probe's 0 - r < threshold holds for every
-    // threshold > 0, so a positive threshold always stops the substep after its first round.
-    const int run = (P.convergence_threshold > 0.0f && rounds > 1) ? 1 : rounds;
+    const int run = roundsRun(rounds);
     launchStamps(d, sp, false, stream);
     if (roundQueue && !colours && nForces == 0 && run <= kMaxQueueRounds) {
         QueueRounds qr{};

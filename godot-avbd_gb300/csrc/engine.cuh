@@ -56,6 +56,7 @@ enum Counter {
     C_PAIRSPILL,      // bodies with more broad-phase partners than the stash holds (pairSpill)
     C_QSOLVE,         // round-loop queue: solve tiles a round (all worlds)
     C_QDUAL,          // round-loop queue: dual tiles a round (all worlds)
+    C_OLDLIVE,        // live manifolds before this step's compaction
     C_TMP,
     C_COUNT
 };
@@ -111,7 +112,9 @@ struct Dev {
     unsigned *qTicket;
     // worlds
     int *wBase, *wCount;    // body range
-    int *wMaxDepth;         // projection: max depth bits per world (positive floats)
+    int *wMan;              // first live manifold per world (+1): live order is world-major
+    int *wOldFirst, *wNewFirst; // compaction: first old / new candidate per world (+1)
+    int *wMaxDepth;         // projection: max depth bits per world, two per world (positive floats)
     int *wStop;             // projection: early-exit flag per world
     int *wBounds;           // Morton scene bounds per world: lo xyz, hi xyz (ordered ints)
     int *wActive;           // projection: movable manifolds per world (0 = skip the world)
@@ -206,5 +209,16 @@ __device__ __forceinline__ int adjInfoSide(int v) { return static_cast<int>(stat
 // In this step's update set (solved, braked, projected).
 __device__ __forceinline__ bool inUpdate(const Dev &d, int g) { return d.upd[g] != 0; }
 constexpr uint8_t kNotUpdated = 10; // colour of a movable body outside the update set
+// Zero the components of `v` on the locked axes (bits 0..2).
+__device__ __forceinline__ void maskLocked(int locks, f3 &v) {
+    if (locks) {
+        if (locks & 1)
+            v.x = 0.0f;
+        if (locks & 2)
+            v.y = 0.0f;
+        if (locks & 4)
+            v.z = 0.0f;
+    }
+}
 
 } // namespace avbdg

@@ -189,6 +189,11 @@ private:
     // device reaches host memory through the host's page tables; else through pinned staging.
     bool roundQueue = false; // AVBDG_QUEUE=1: the round loop as one tile-queue launch where it applies
     bool bruteAllowed = true; // AVBDG_NO_BRUTE=1: candidate pairs always from the tree walk
+    bool worldAllowed = true; // AVBDG_NO_WORLD=1: the step's second half always as separate launches
+    // The live manifolds are in world order (or there is one world). Stores of up to this many bodies keep
+    // them so: larger ones hold too many worlds to be stepped a cluster a world.
+    static constexpr int kWorldMajorBodies = 65536;
+    bool liveByWorld = true;
     bool stepPending = false; // stepEnqueue ran, stepFinish has not
     int pendingLaunches = 0;  // kernels the pending step launched
     bool directIo = false;
@@ -214,6 +219,10 @@ private:
         bool adjAtStart = false, anyTree = false, rebuild = false, forces = false, greedy = false;
         bool multiWorld = false, round = false;
         bool brute = false; // pairs by the all-pairs test within each world instead of the tree
+        // The step's second half as one launch, a cluster per world: worlds and the largest one's
+        // bodies, each rounded up to a power of two (0: separate launches).
+        int worldCount = 0, worldBodies = 0;
+        bool worldMajor = false; // the compaction leaves the live manifolds in world order
         std::string key() const;
     };
     struct Graph {
@@ -234,9 +243,13 @@ private:
     void dropGraphs();
     void recordPhase(cudaEvent_t e);
     int broadPhase(const StepParams &sp, const StepPlan &plan);
-    int warmstartAndSelect(const StepParams &sp);
+    int warmstartAndSelect(const StepParams &sp, const StepPlan &plan);
+    void sortLiveByWorld();
     void projectContacts(const StepParams &sp, bool positions, real window);
     void runSubstep(const StepParams &sp, int rounds, bool idle);
+    int roundsRun(int rounds) const;
+    int newtonRoundsOf(int rounds) const;
+    void runWorlds(const StepParams &sp, const StepPlan &plan);
     int finishStep();
     bool needGreedy() const;
 };

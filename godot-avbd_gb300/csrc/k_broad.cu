@@ -572,6 +572,7 @@ __global__ void candTotalKernel(Dev d) {
         c = d.MM;
     }
     d.ctr[C_CAND] = c;
+    d.ctr[C_OLDLIVE] = d.ctr[C_LIVE];
 }
 
 } // namespace

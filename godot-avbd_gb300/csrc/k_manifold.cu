@@ -13,6 +13,7 @@
 #include "narrow.cuh"
 #include "narrow_round.cuh"
 #include "prims.cuh"
+#include "project.cuh"
 
 namespace avbdg {
 
@@ -100,12 +101,6 @@ __global__ void adjTotalKernel(Dev d) {
 }
 
 // ---- manifold initialize (ManifoldStore::initialize, manifold.cpp:237-435) ----
-
-// mul(basis, v) with the basis stored as rows.
-__device__ __forceinline__ f3 basisMul(f3 r0, f3 r1, f3 r2, f3 v) {
-    return f3{(r0.x * v.x + r0.y * v.y) + r0.z * v.z, (r1.x * v.x + r1.y * v.y) + r1.z * v.z,
-              (r2.x * v.x + r2.y * v.y) + r2.z * v.z};
-}
 
 // ROUND: the store holds spheres or cylinders, whose sampled paths need kilobytes of local memory
 // per thread; box-only stores run the variant without them.
@@ -339,7 +334,7 @@ __device__ __forceinline__ void manifoldCompactRun(const Dev &d, const int *flag
         const int i = static_cast<int>(t - static_cast<T>(c) * static_cast<T>(cand));
         if (!flags[i])
             continue;
-        const int r = rank[i];
+        const int r = rank ? rank[i] : flags[i] - 1; // one world: its rank; several: its place
         const int n = S.count[i];
         const int2 dorm = S.dormant[i];
         if (c == 0) {
@@ -384,24 +379,47 @@ __global__ void manifoldCompactKernel(Dev d, const int *flags, const int *rank) 
         manifoldCompactRun<unsigned long long>(d, flags, rank, cand);
 }
 
-// ---- rebase (ManifoldStore::rebase, manifold.cpp:448-461) ----
-__device__ __forceinline__ void rebaseAt(Dev d, StepParams p, int m) {
-    if (m >= d.ctr[C_LIVE])
-        return;
-    const ManifoldBuf L = d.live;
-    const int2 ab = L.ab[m];
-    const f3 xa = xyz(d.x[ab.x]), xb = xyz(d.x[ab.y]);
-    const q4 qa = asq(d.q[ab.x]), qb = asq(d.q[ab.y]);
-    const f3 r0 = xyz(L.b0[m]), r1 = xyz(L.b1[m]), r2 = xyz(L.b2[m]);
-    const int n = L.count[m];
-    for (int c = 0; c < n; c++) {
-        const int ci = cslot(d, m, c);
-        const f3 pA = add(xa, qrot(qa, xyz(L.rA[ci])));
-        const f3 pB = add(xb, qrot(qb, xyz(L.rB[ci])));
-        f3 C0 = add(basisMul(r0, r1, r2, sub(pA, pB)), f3{COLLISION_MARGIN, 0, 0});
-        if (C0.x < -p.maxPen)
-            C0.x = -p.maxPen;
-        L.C0[ci] = f4(C0, 0.0f);
+// ---- world-major order ----
+// Candidates are the old live manifolds, then the new ones, each part ordered by world (new pairs
+// are sorted by list position, the old ones were left so by the step before). A world's survivors
+// are its old ones, then its new ones, after those of the worlds before it. (Large
+// stores go without: on the 4096-world batch the order took the dual pass from 133 to 126 us a round,
+// but the brake's dataflow from 130 to 160 us a sweep and the passes below cost 13 us a step.)
+
+// Where each world's candidates begin in the old part (wOldFirst) and in the new one (wNewFirst);
+// entry [worlds] of each is the part's end.
+__global__ void worldFirstKernel(Dev d) {
+    pdlWait();
+    pdlTrigger();
+    const int cand = d.ctr[C_CAND], old = min(d.ctr[C_OLDLIVE], cand), nWorlds = d.ctr[C_WORLDS];
+    const int2 *ab = d.stage.ab;
+    // Candidate i begins the worlds after its predecessor's up to its own; the ends' are the part's.
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    for (int k = i; k < cand + 2; k += gridDim.x * blockDim.x) {
+        const bool isNew = k > old; // slots 0..old: the old part and its end; old+1..cand+1: the new one's
+        const int first = isNew ? old : 0, end = isNew ? cand : old, at = isNew ? k - 1 : k;
+        const int from = at == first ? 0 : d.meta[ab[at - 1].x].x + 1;
+        const int to = at == end ? nWorlds : d.meta[ab[at].x].x;
+        int *out = isNew ? d.wNewFirst : d.wOldFirst;
+        for (int w = from; w <= to; w++)
+            out[w] = at;
+    }
+}
+
+// Each candidate's place (flags: 0 for one that is dropped, else its place + 1) and each world's range.
+__global__ void worldRankKernel(Dev d, const int *rank, int *flags) {
+    pdlWait();
+    pdlTrigger();
+    const int cand = d.ctr[C_CAND], old = min(d.ctr[C_OLDLIVE], cand), live = d.ctr[C_LIVE], nWorlds = d.ctr[C_WORLDS];
+    const auto kept = [&](int i) { return i < cand ? rank[i] : live; }; // survivors before candidate i
+    const int keptOld = kept(old);
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < cand || i <= nWorlds; i += gridDim.x * blockDim.x) {
+        if (i <= nWorlds)
+            d.wMan[i] = kept(d.wOldFirst[i]) + kept(d.wNewFirst[i]) - keptOld;
+        if (i >= cand || !flags[i])
+            continue;
+        const int w = d.meta[d.stage.ab[i].x].x;
+        flags[i] = 1 + (i < old ? rank[i] + kept(d.wNewFirst[w]) - keptOld : kept(d.wOldFirst[w + 1]) + rank[i] - keptOld);
     }
 }
 
@@ -533,12 +551,59 @@ void launchManifoldInit(const Dev &d, const StepParams &p, bool round, int block
         launchK(manifoldInitKernel<false>, divUp(d.MM, block), block, 0, s, d, p);
 }
 
-void launchManifoldCompact(const Dev &d, cudaStream_t s) {
+void launchManifoldCompact(const Dev &d, bool worldMajor, cudaStream_t s) {
     scanExclusive(d.mActive, d.pairValid, d.MM, d.ctr + C_CAND, d.ctr + C_LIVE, d.scanScratch, s);
+    if (worldMajor) {
+        ++launchCount(); launchK(worldFirstKernel, residentGrid(worldFirstKernel, kThreads, grid(d.MM + 2)), kThreads, 0, s, d);
+        ++launchCount();
+        launchK(worldRankKernel, residentGrid(worldRankKernel, kThreads, grid(d.MM > d.WW ? d.MM : d.WW + 1)), kThreads, 0, s, d,
+                d.pairValid, d.mActive);
+    }
     ++launchCount();
     const int blocks = residentGrid(reinterpret_cast<const void *>(manifoldCompactKernel), kThreads, 0,
                                     divUp(d.MM * kMaxContacts, kThreads));
-    launchK(manifoldCompactKernel, blocks, kThreads, 0, s, d, d.mActive, d.pairValid);
+    launchK(manifoldCompactKernel, blocks, kThreads, 0, s, d, d.mActive, worldMajor ? nullptr : d.pairValid);
+}
+
+// The live manifolds to the staging buffer and back to their new places (rare: a store that starts to
+// keep its live order by world).
+void launchManifoldPermute(const Dev &d, const std::vector<int> &places, cudaStream_t s) {
+    const size_t n = places.size();
+    if (n == 0)
+        return;
+    std::vector<int> flags(n);
+    for (size_t i = 0; i < n; i++)
+        flags[i] = places[i] + 1;
+    const int count = static_cast<int>(n);
+    cudaMemcpyAsync(d.mActive, flags.data(), sizeof(int) * n, cudaMemcpyHostToDevice, s);
+    cudaMemcpyAsync(d.ctr + C_CAND, &count, sizeof(int), cudaMemcpyHostToDevice, s);
+    const auto cp = [&](void *to, const void *from, size_t bytes) { cudaMemcpyAsync(to, from, bytes, cudaMemcpyDeviceToDevice, s); };
+    const ManifoldBuf &L = d.live, &S = d.stage;
+    cp(S.ab, L.ab, sizeof(int2) * n);
+    cp(S.b0, L.b0, sizeof(real4) * n);
+    cp(S.b1, L.b1, sizeof(real4) * n);
+    cp(S.b2, L.b2, sizeof(real4) * n);
+    cp(S.count, L.count, sizeof(int) * n);
+    cp(S.dormant, L.dormant, sizeof(int2) * n);
+    for (int c = 0; c < kMaxContacts; c++) {
+        const size_t at = static_cast<size_t>(c) * d.MM;
+        cp(S.key + at, L.key + at, sizeof(int) * n);
+        for (auto pr : {std::make_pair(S.rA, L.rA), std::make_pair(S.rB, L.rB), std::make_pair(S.C0, L.C0),
+                        std::make_pair(S.k, L.k), std::make_pair(S.lam, L.lam)})
+            cp(pr.first + at, pr.second + at, sizeof(real4) * n);
+        if (d.ARM) {
+            cp(S.armA + at, L.armA + at, sizeof(real4) * n);
+            cp(S.armB + at, L.armB + at, sizeof(real4) * n);
+        }
+    }
+    if (d.ARM) {
+        cp(S.capA, L.capA, sizeof(real4) * n);
+        cp(S.capB, L.capB, sizeof(real4) * n);
+        cp(S.armFlag, L.armFlag, sizeof(uint8_t) * n);
+    }
+    ++launchCount();
+    launchK(manifoldCompactKernel, divUp(count * kMaxContacts, kThreads), kThreads, 0, s, d, d.mActive, static_cast<const int *>(nullptr));
+    cudaStreamSynchronize(s); // the host arrays above are read until here
 }
 
 void launchRebase(const Dev &d, const StepParams &p, cudaStream_t s) {

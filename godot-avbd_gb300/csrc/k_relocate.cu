@@ -179,7 +179,7 @@ void launchRelocateWorlds(const Dev &d, int nOld, int nNew, int nForces, const i
     // Live manifolds: stage with new body slots, then the step's stable compaction into live.
     cudaMemcpyAsync(d.ctr + C_CAND, d.ctr + C_LIVE, sizeof(int), cudaMemcpyDeviceToDevice, s);
     ++launchCount(); launchK(manifoldRelocateKernel, grid(d.MM), kThreads, 0, s, d, slotMap);
-    launchManifoldCompact(d, s);
+    launchManifoldCompact(d, false, s);
 
     // Forces: flags + exclusive rank, then a stable scatter of every field.
     if (nForces > 0) {

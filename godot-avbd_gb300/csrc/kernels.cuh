@@ -1,6 +1,8 @@
 // Host-side launchers of the step's kernels (one function per kernel or kernel group).
 #pragma once
 
+#include <vector>
+
 #include "engine.cuh"
 
 namespace avbdg {
@@ -35,7 +37,11 @@ void launchFilterAcquire(const Dev &d, cudaStream_t s);
 // ---- manifolds and adjacency (k_manifold.cu) ----
 void launchAdjacency(const Dev &d, cudaStream_t s);
 void launchManifoldInit(const Dev &d, const StepParams &p, bool round, int block, cudaStream_t s);
-void launchManifoldCompact(const Dev &d, cudaStream_t s);
+// `worldMajor`: survivors are ordered by world (each world's own order kept), world w's at
+// [wMan[w], wMan[w + 1]).
+void launchManifoldCompact(const Dev &d, bool worldMajor, cudaStream_t s);
+// Moves the live manifolds to places places[m] (given on the host, a permutation of 0..n-1).
+void launchManifoldPermute(const Dev &d, const std::vector<int> &places, cudaStream_t s);
 void launchRebase(const Dev &d, const StepParams &p, cudaStream_t s);
 void launchForceInit(const Dev &d, const StepParams &p, bool forces, cudaStream_t s);
 
@@ -75,6 +81,21 @@ void launchOverflowApply(const Dev &d, const StepParams &p, cudaStream_t s);
 // bodies are all overflow or static. `decay` < 1 scales penalties first (dual-only rounds).
 void launchDual(const Dev &d, const StepParams &p, bool stamps, real decay, int block, cudaStream_t s);
 void launchForceDual(const Dev &d, const StepParams &p, bool forces, cudaStream_t s);
+
+// ---- the step from the brake to the rebase, a cluster per world (k_world.cu) ----
+struct WorldRun {
+    int substeps, rounds, newtonRounds;
+    real dt;            // of a substep (the brake's window counts them down)
+    real tolerance;     // projection: a pass whose deepest patch is within it is the last
+    bool brake, project, colours, multiWorld;
+    unsigned rowBytes, smemBytes; // set by the launch
+};
+int worldTeamMax();
+// Whether a store of up to `worlds` worlds of up to `bodies` bodies, with about `density` manifolds a
+// body, is stepped this way.
+bool worldsTake(int worlds, int bodies, double density);
+// `worlds`: at least the store's worlds; `bodies`: at least the largest one's.
+void launchWorlds(const Dev &d, const StepParams &p, const WorldRun &run, int worlds, int bodies, cudaStream_t s);
 
 // ---- projection (k_proj.cu) ----
 // projectionActive per world and the brake candidates (manifolds with an open gap).

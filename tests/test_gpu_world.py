@@ -1,0 +1,93 @@
+"""The step's second half as one launch, a cluster per world: worlds around its limits (bodies a
+CTA, contact tasks, worlds whose parts do not fit in shared memory, many worlds in one store) against
+the oracle, bit for bit."""
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def run(api, capi, descs, steps, params=None, interleaved=None, room=0):
+    p = api.default_params()
+    for k, v in (params or {}).items():
+        setattr(p, k, v)
+    w = capi.World(api, p, max_bodies=max(len(descs), room))
+    w.add_bodies(descs)
+    out = []
+    for _ in range(steps):
+        if interleaved:
+            w.step_interleaved(*interleaved)
+        else:
+            w.step()
+        out.append(w.state())
+    return out
+
+
+def same(a, b):
+    return all(np.array_equal(x, y, equal_nan=True) for s, t in zip(a, b) for x, y in zip(s, t))
+
+
+def heap(capi, n, seed, spread=1.0):
+    """`n` boxes of unequal size and random orientation in a loose heap on a ground."""
+    rng = np.random.default_rng(seed)
+    size = rng.uniform(0.4, 1.2, (n, 3))
+    q = rng.normal(size=(n, 4))
+    q /= np.linalg.norm(q, axis=1, keepdims=True)
+    side = max(1, int(np.ceil((n / 3.0) ** 0.5)))
+    i = np.arange(n)
+    pos = np.stack([spread * (i % side), spread * (i // side % side), 0.8 + 1.1 * (i // (side * side))], 1)
+    pos += rng.uniform(-0.05, 0.05, pos.shape)
+    return capi.make_body_descs(np.concatenate([[[80, 80, 1]], size]), [0.0] + [1.0] * n, 0.5,
+                                np.concatenate([[[0, 0, -0.5]], pos]), np.concatenate([[[0, 0, 0, 1]], q]),
+                                np.concatenate([[[0, 0, 0]], rng.uniform(-1, 1, (n, 3))]))
+
+
+# One CTA, two, the odd sizes around a CTA's share of the bodies, the largest cluster.
+@pytest.mark.parametrize("n", [1, 2, 23, 24, 25, 49, 97, 193, 385, 700])
+def test_sizes(pkg, gpu, oracle, n):
+    capi = pkg.capi
+    d = heap(capi, n, n)
+    assert same(run(gpu, capi, d, 25), run(oracle, capi, d, 25))
+
+
+# Bodies inside one another: far more manifolds a body than the shared-memory form holds, in the first
+# step (before any count is known) and after.
+@pytest.mark.parametrize("n,spread", [(150, 0.25), (260, 0.12)])
+def test_dense_world_does_not_fit(pkg, gpu, oracle, n, spread):
+    capi = pkg.capi
+    d = heap(capi, n, 3, spread)
+    room = 16384  # the store is sized by this: eight manifolds and sixteen pairs a body
+    assert same(run(gpu, capi, d, 6, room=room), run(oracle, capi, d, 6))
+
+
+@pytest.mark.parametrize("params,interleaved", [
+    ({"jacobian_rebuild_distance": 0.02}, None), ({"jacobian_rebuild_distance": 0.05, "dt": 1 / 120}, (2, 3)),
+    ({"position_projection": 0}, None), ({"speculative_margin": 0.0}, None), ({"newton_ratio": 0.5}, None),
+    ({"adaptive_beta": 1, "iterations": 3}, (3, 2))])
+def test_options(pkg, gpu, oracle, params, interleaved):
+    capi = pkg.capi
+    d = heap(capi, 120, 9)
+    assert same(run(gpu, capi, d, 20, params, interleaved), run(oracle, capi, d, 20, params, interleaved))
+
+
+def test_many_worlds_added_and_removed(pkg, gpu):
+    """A store that starts too large to be kept in world order, then loses worlds until it is, then gains
+    one: each world equals the same world alone."""
+    capi = pkg.capi
+    worlds, n = 500, 140
+    b = capi.Batch(gpu.lib, max_worlds=worlds, max_bodies=worlds * (n + 1))
+    kinds = [heap(capi, n, s) for s in range(5)]
+    add = lambda d: (b._api.check(b.fn["batch_add_world"](b.handle, len(d), d, 0, None, capi.C.byref(capi.C.c_int()))),
+                     b.sizes.append(len(d)))
+    for w in range(worlds):
+        add(kinds[w % 5])
+    b.step(8)
+    b.remove_worlds([w for w in range(worlds) if w % 10])
+    b.step(8)
+    add(kinds[0])
+    b.step(8)
+    alone = [run(gpu, capi, d, 24) for d in kinds]
+    for w in range(0, 50, 7):
+        assert same([b.state(w)], [alone[w * 10 % 5][23]])
+    assert same([b.state(50)], [alone[0][7]])
