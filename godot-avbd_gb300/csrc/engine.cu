@@ -910,6 +910,8 @@ Engine::StepPlan Engine::planStep(int mode, int substeps, int rounds) {
             plan.worldBodies = bodies;
         }
     }
+    if (worldAllowed && worlds() == 1 && plan.anyTree && most <= worldPairsMost())
+        plan.front = most;
     return plan;
 }
 
@@ -935,9 +937,9 @@ void Engine::sortLiveByWorld() {
 
 std::string Engine::StepPlan::key() const {
     char buf[128];
-    std::snprintf(buf, sizeof(buf), "%d/%d/%d/%d%d%d%d%d%d%d%d%d/%d/%d", mode, substeps, rounds, adjAtStart ? 1 : 0,
+    std::snprintf(buf, sizeof(buf), "%d/%d/%d/%d%d%d%d%d%d%d%d%d/%d/%d/%d", mode, substeps, rounds, adjAtStart ? 1 : 0,
                   anyTree ? 1 : 0, rebuild ? 1 : 0, forces ? 1 : 0, greedy ? 1 : 0, multiWorld ? 1 : 0,
-                  round ? 1 : 0, brute ? 1 : 0, worldMajor ? 1 : 0, worldCount, worldBodies);
+                  round ? 1 : 0, brute ? 1 : 0, worldMajor ? 1 : 0, worldCount, worldBodies, front);
     return buf;
 }
 
@@ -951,6 +953,18 @@ void Engine::recordPhase(cudaEvent_t e) {
 int Engine::broadPhase(const StepParams &sp, const StepPlan &plan) {
     if (plan.adjAtStart)
         launchAdjacency(d, stream);
+    if (plan.front) {
+        if (plan.rebuild) { // the tree's codes and order are dumped on the reference's schedule
+            launchAabb(d, sp, stream);
+            launchRebuildTree(d, plan.multiWorld, stream);
+        }
+        beginSpan();
+        launchWorldPairs(d, sp, plan.front, stream);
+        endSpan(kTraverse);
+        if (sp.sleepFrames > 0)
+            launchSleepWakePairs(d, stream);
+        return AVBDG_OK;
+    }
     launchAabb(d, sp, stream);
     if (!plan.anyTree) {
         cudaMemsetAsync(d.ctr + C_PAIRS, 0, sizeof(int), stream);
@@ -1146,11 +1160,20 @@ int Engine::runPlan(const StepPlan &plan) {
 // warmstartForces + selectUpdateBodies (solver_solve.cpp:31-105, 263-424).
 int Engine::warmstartAndSelect(const StepParams &sp, const StepPlan &plan) {
     launchForceInit(d, sp, nForces > 0, stream);
-    beginSpan();
-    launchManifoldInit(d, sp, nRound > 0, tuned.narrow, stream);
-    endSpan(kNarrow);
-    launchManifoldCompact(d, plan.worldMajor, stream);
-    launchAdjacency(d, stream);
+    if (plan.front) {
+        const bool select = sp.sleepFrames == 0 && !needGreedy();
+        beginSpan();
+        launchWorldContacts(d, sp, nRound > 0, select, plan.front, stream);
+        endSpan(kNarrow);
+        if (select)
+            return AVBDG_OK;
+    } else {
+        beginSpan();
+        launchManifoldInit(d, sp, nRound > 0, tuned.narrow, stream);
+        endSpan(kNarrow);
+        launchManifoldCompact(d, plan.worldMajor, stream);
+        launchAdjacency(d, stream);
+    }
     if (sp.sleepFrames > 0)
         launchSleepSelect(d, sp, stream);
     launchContactOnly(d, stream);

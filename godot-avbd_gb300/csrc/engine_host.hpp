@@ -222,6 +222,7 @@ private:
         // The step's second half as one launch, a cluster per world: worlds and the largest one's
         // bodies, each rounded up to a power of two (0: separate launches).
         int worldCount = 0, worldBodies = 0;
+        int front = 0; // the step's first half as two launches of one cluster: the world's bodies (0: separate)
         bool worldMajor = false; // the compaction leaves the live manifolds in world order
         std::string key() const;
     };

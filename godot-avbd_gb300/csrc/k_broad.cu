@@ -9,6 +9,9 @@
 // larger list index, and per-body segments are sorted, so the sorted key list equals the
 // reference's sorted, de-duplicated sweepPairs bit for bit.
 
+#include <algorithm>
+
+#include "cluster.cuh"
 #include "kernels.cuh"
 #include "prims.cuh"
 
@@ -25,14 +28,9 @@ __device__ __forceinline__ int orderedInt(real f) {
 }
 __device__ __forceinline__ real orderedFloat(int i) { return bitsf(i >= 0 ? i : i ^ 0x7fffffff); }
 
-// Swept AABB (solver_broadphase.cpp:103-122) over the tight box bound (rigid.cpp:83-106).
-__global__ void aabbKernel(Dev d, StepParams p) {
-    pdlWait();
-    pdlTrigger();
-    const int n = d.ctr[C_BODIES];
-    const int g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= n || d.meta[g].x < 0)
-        return;
+// Swept AABB (solver_broadphase.cpp:103-122) over the tight box bound (rigid.cpp:83-106): centre and
+// half extents.
+__device__ __forceinline__ void sweptBox(const Dev &d, const StepParams &p, int g, f3 &c, f3 &half) {
     const real4 x4 = d.x[g];
     const real4 v4 = d.v[g];
     const real4 s4 = d.size[g];
@@ -49,8 +47,19 @@ __global__ void aabbKernel(Dev d, StepParams p) {
         disp = add(disp, f3{0, 0, v4.w * cdt * cdt});
     const real rotSweep = s4.w * length(xyz(d.w[g])) * cdt;
     const real grow = rotSweep + p.specMargin;
-    const f3 c = add(xyz(x4), scale(disp, 0.5f));
-    const f3 half = add(add(tight, scale(vabs(disp), 0.5f)), f3{grow, grow, grow});
+    c = add(xyz(x4), scale(disp, 0.5f));
+    half = add(add(tight, scale(vabs(disp), 0.5f)), f3{grow, grow, grow});
+}
+
+__global__ void aabbKernel(Dev d, StepParams p) {
+    pdlWait();
+    pdlTrigger();
+    const int n = d.ctr[C_BODIES];
+    const int g = blockIdx.x * blockDim.x + threadIdx.x;
+    if (g >= n || d.meta[g].x < 0)
+        return;
+    f3 c, half;
+    sweptBox(d, p, g, c, half);
     d.aabbC[g] = f4(c, 0.0f);
     d.aabbH[g] = f4(half, 0.0f);
 }
@@ -504,17 +513,8 @@ __global__ void pairTotalKernel(Dev d) {
     d.ctr[C_PAIRS] = t;
 }
 
-// pairOverlaps (solver_broadphase.cpp:30-65): bounds, layer/mask, not constrained, not both static.
-__device__ __forceinline__ void filterAt(Dev d, int k) {
-    const int np = d.ctr[C_PAIRS];
-    if (k >= np)
-        return;
-    const uint64_t key = d.pairs[k];
-    const int a = d.lpToBody[static_cast<int>(key >> 32)];
-    const int b = d.lpToBody[static_cast<int>(key & 0xffffffffu)];
-    const real4 ac = d.aabbC[a], ah = d.aabbH[a], bc = d.aabbC[b], bh = d.aabbH[b];
-    const bool bounds = overlapClosed(f3{ac.x - ah.x, ac.y - ah.y, ac.z - ah.z}, f3{ac.x + ah.x, ac.y + ah.y, ac.z + ah.z},
-                                      f3{bc.x - bh.x, bc.y - bh.y, bc.z - bh.z}, f3{bc.x + bh.x, bc.y + bh.y, bc.z + bh.z});
+// Layers and masks, not constrained, not both static (solver_broadphase.cpp:30-65 beside the bounds).
+__device__ __forceinline__ bool pairAllowed(const Dev &d, int a, int b) {
     const int4 ma = d.meta[a], mb = d.meta[b];
     const bool layers = ((static_cast<uint32_t>(ma.y) & static_cast<uint32_t>(mb.z)) != 0) ||
                         ((static_cast<uint32_t>(mb.y) & static_cast<uint32_t>(ma.z)) != 0);
@@ -531,9 +531,22 @@ __device__ __forceinline__ void filterAt(Dev d, int k) {
                 break;
             }
     }
-    d.pairValid[k] = (bounds && layers && !constrained && !bothStatic) ? 1 : 0;
+    return layers && !constrained && !bothStatic;
 }
 
+// pairOverlaps (solver_broadphase.cpp:30-65): bounds, layer/mask, not constrained, not both static.
+__device__ __forceinline__ void filterAt(Dev d, int k) {
+    const int np = d.ctr[C_PAIRS];
+    if (k >= np)
+        return;
+    const uint64_t key = d.pairs[k];
+    const int a = d.lpToBody[static_cast<int>(key >> 32)];
+    const int b = d.lpToBody[static_cast<int>(key & 0xffffffffu)];
+    const real4 ac = d.aabbC[a], ah = d.aabbH[a], bc = d.aabbC[b], bh = d.aabbH[b];
+    const bool bounds = overlapClosed(f3{ac.x - ah.x, ac.y - ah.y, ac.z - ah.z}, f3{ac.x + ah.x, ac.y + ah.y, ac.z + ah.z},
+                                      f3{bc.x - bh.x, bc.y - bh.y, bc.z - bh.z}, f3{bc.x + bh.x, bc.y + bh.y, bc.z + bh.z});
+    d.pairValid[k] = bounds && pairAllowed(d, a, b) ? 1 : 0;
+}
 __global__ void filterKernel(Dev d) {
     pdlWait();
     pdlTrigger();
@@ -574,6 +587,147 @@ __global__ void candTotalKernel(Dev d) {
     d.ctr[C_CAND] = c;
     d.ctr[C_OLDLIVE] = d.ctr[C_LIVE];
 }
+
+// ---- one world's candidate pairs, filter and acquisition in one launch ----
+//
+// For a store of one world of up to some thousand bodies the separate launches (bounds, pair counts, a
+// scan, pairs, their sort, filter, a scan, acquisition) are ~20 fixed costs of a few microseconds. Here a
+// cluster does them all: every CTA holds the world's boxes in shared memory, a warp tests one body
+// against the bodies before it in slots, 32 at a time in list order, so its partners come out sorted;
+// counts are scanned by every CTA reading all of them (clusterShare).
+constexpr int kPairThreads = 512;
+
+struct Box {
+    real4 lo, hi;
+};
+
+__global__ void __launch_bounds__(kPairThreads, 1)
+        worldPairsKernel(const __grid_constant__ Dev d, const __grid_constant__ StepParams p) {
+    pdlWait();
+    pdlTrigger();
+    extern __shared__ __align__(32) unsigned char smem[];
+    __shared__ int warpSums[kPairThreads / 32];
+    Box *box = reinterpret_cast<Box *>(smem);
+    const int rank = clusterRank(), size = clusterSize(), lane = threadIdx.x & 31;
+    const int n = d.ctr[C_BODIES];
+    for (int g = threadIdx.x; g < n; g += kPairThreads) {
+        f3 c, h;
+        sweptBox(d, p, g, c, h);
+        box[g] = Box{mk4(c.x - h.x, c.y - h.y, c.z - h.z, 0.0f), mk4(c.x + h.x, c.y + h.y, c.z + h.z, 0.0f)};
+        if ((g >> 5) % size == rank) {
+            d.aabbC[g] = f4(c, 0.0f);
+            d.aabbH[g] = f4(h, 0.0f);
+        }
+    }
+    __syncthreads();
+    const int warp = rank + size * static_cast<int>(threadIdx.x >> 5), warps = size * (kPairThreads / 32);
+    // The partners of body g with a larger list position are the bodies in smaller slots, nearest first.
+    const auto partners = [&](int g, auto &&each) { // each(hit, rank among the hits, slot); returns their number
+        const real4 lo = box[g].lo, hi = box[g].hi;
+        int found = 0;
+        for (int b0 = g - 1; b0 >= 0; b0 -= 32) {
+            const int b = b0 - lane;
+            bool hit = false;
+            if (b >= 0) {
+                const real4 bl = box[b].lo, bh = box[b].hi;
+                hit = overlapClosed(f3{lo.x, lo.y, lo.z}, f3{hi.x, hi.y, hi.z}, f3{bl.x, bl.y, bl.z}, f3{bh.x, bh.y, bh.z});
+            }
+            const unsigned hits = __ballot_sync(0xffffffffu, hit);
+            if (hits) {
+                each(hit, found + __popc(hits & ((1u << lane) - 1u)), b);
+                found += __popc(hits);
+            }
+        }
+        return found;
+    };
+    int *counts = d.pairSpill, *valid = d.solveFail; // scratch per list position
+    for (int g = warp; g < n; g += warps) {
+        const int lp = n - 1 - g;
+        int *stash = d.pairStash + static_cast<size_t>(lp) * kPairStash;
+        const int found = partners(g, [&](bool hit, int at, int b) {
+            if (hit && at < kPairStash)
+                stash[at] = b;
+        });
+        if (lane == 0)
+            counts[lp] = found;
+    }
+    clusterSync(size);
+    // Pairs in key order: this CTA's list positions, a warp each; the filter on the way.
+    const Share share = clusterShare(counts, n, rank, size, warpSums);
+    for (int tile = share.lo, run = share.before; tile < share.hi; tile += kPairThreads) {
+        const int mine = tile + static_cast<int>(threadIdx.x);
+        int all;
+        const int start = run + blockPrefix(mine < share.hi ? counts[mine] : 0, warpSums, all);
+        if (mine < share.hi)
+            d.pairStart[mine] = start;
+        run += all;
+    }
+    __syncthreads();
+    for (int lp = share.lo + static_cast<int>(threadIdx.x >> 5); lp < share.hi; lp += kPairThreads / 32) {
+        const int g = n - 1 - lp, start = d.pairStart[lp], found = counts[lp];
+        int allowed = 0;
+        const auto emit = [&](bool on, int at, int b) {
+            bool ok = false;
+            if (on && start + at < d.PP) {
+                d.pairs[start + at] = (static_cast<uint64_t>(lp) << 32) | static_cast<uint32_t>(n - 1 - b);
+                ok = pairAllowed(d, g, b);
+                d.pairValid[start + at] = ok ? 1 : 0;
+            }
+            allowed += __popc(__ballot_sync(0xffffffffu, ok));
+        };
+        if (found <= kPairStash) {
+            const int *stash = d.pairStash + static_cast<size_t>(lp) * kPairStash;
+            for (int at = lane; at - lane < found; at += 32)
+                emit(at < found, at, at < found ? stash[at] : 0);
+        } else {
+            partners(g, emit);
+        }
+        if (lane == 0)
+            valid[lp] = allowed;
+    }
+    clusterSync(size);
+    // New manifolds after the live ones, in key order.
+    const Share fresh = clusterShare(valid, n, rank, size, warpSums);
+    const int live = d.ctr[C_LIVE];
+    int *starts = d.adjFill; // scratch per list position (the adjacency that follows resets it)
+    for (int tile = fresh.lo, run = fresh.before; tile < fresh.hi; tile += kPairThreads) {
+        const int mine = tile + static_cast<int>(threadIdx.x);
+        int all;
+        const int start = run + blockPrefix(mine < fresh.hi ? valid[mine] : 0, warpSums, all);
+        if (mine < fresh.hi)
+            starts[mine] = start;
+        run += all;
+    }
+    __syncthreads();
+    for (int lp = fresh.lo + static_cast<int>(threadIdx.x >> 5); lp < fresh.hi; lp += kPairThreads / 32) {
+        const int start = d.pairStart[lp], found = counts[lp];
+        int m = live + starts[lp];
+        for (int at = lane; at - lane < found; at += 32) {
+            const int k = start + at;
+            const bool ok = at < found && k < d.PP && d.pairValid[k];
+            const unsigned oks = __ballot_sync(0xffffffffu, ok);
+            const int to = m + __popc(oks & ((1u << lane) - 1u));
+            if (ok && to < d.MM) {
+                d.live.ab[to] = make_int2(n - 1 - lp, n - 1 - static_cast<int>(d.pairs[k] & 0xffffffffu));
+                d.live.count[to] = 0;
+                d.live.dormant[to] = make_int2(0, 0);
+            }
+            m += __popc(oks);
+        }
+    }
+    if (rank == 0 && threadIdx.x == 0) {
+        if (share.total > d.PP)
+            atomicOr(&d.ctr[C_ERRORS], kErrPairs);
+        d.ctr[C_PAIRS] = min(share.total, d.PP);
+        if (live + fresh.total > d.MM)
+            atomicOr(&d.ctr[C_ERRORS], kErrManifolds);
+        d.ctr[C_CAND] = min(live + fresh.total, d.MM);
+        d.ctr[C_OLDLIVE] = live;
+    }
+}
+
+int g_pairTeam = 0;
+constexpr int kPairSmem = 220 * 1024; // of a CTA; the world's boxes are in it
 
 } // namespace
 
@@ -635,6 +789,29 @@ void launchFilterAcquire(const Dev &d, cudaStream_t s) {
     scanExclusive(d.pairValid, d.mActive, d.PP, d.ctr + C_PAIRS, d.ctr + C_TMP, d.scanScratch, s);
     ++launchCount(); launchK(acquireKernel, residentGrid(acquireKernel, kThreads, grid(d.PP)), kThreads, 0, s, d, d.pairValid, d.mActive);
     ++launchCount(); launchK(candTotalKernel, 1, 1, 0, s, d);
+}
+
+static int pairTeamMax() {
+    if (g_pairTeam == 0)
+        g_pairTeam = allowTeam(reinterpret_cast<const void *>(worldPairsKernel), kPairThreads, kPairSmem);
+    return g_pairTeam;
+}
+
+// The all-pairs test grows with the square of the bodies, the tree does not. Measured, microseconds a
+// step with this form of the first half and without: 421 bodies 236 / 317, 2001 (pile) 513 / 578, 2521
+// (walls) 568 / 579, 2593 (lattice) 487 / 499, 3201: 527 / 512, 4001 (pile) 762 / 712.
+int worldPairsMost() {
+    pairTeamMax();
+    return std::min(2600, kPairSmem / static_cast<int>(sizeof(Box)));
+}
+
+void launchWorldPairs(const Dev &d, const StepParams &p, int bodies, cudaStream_t s) {
+    int team = 1;
+    while (team < pairTeamMax() && team * 24 < bodies)
+        team *= 2;
+    const TeamLaunch l(team, 1, kPairThreads, sizeof(Box) * static_cast<size_t>(bodies), s);
+    ++launchCount();
+    cudaLaunchKernelEx(&l.cfg, worldPairsKernel, d, p);
 }
 
 } // namespace avbdg

@@ -8,6 +8,7 @@
 
 #include <cmath>
 
+#include "cluster.cuh"
 #include "forces.cuh"
 #include "kernels.cuh"
 #include "narrow.cuh"
@@ -74,6 +75,16 @@ __global__ void adjFillKernel(Dev d) {
 // Each entry's other body and side, once per adjacency build, so the per-round passes need no
 // load of the force's or manifold's body pair to find them; and each manifold side's entry, where
 // its block stamp is stored, so a body's stamps lie contiguous in its adjacency range.
+__device__ __forceinline__ void adjInfoAt(const Dev &d, int g, int e, int seq) {
+    const int nf = d.ctr[C_FORCES];
+    const int2 ab = seq < nf ? d.fAB[nf - 1 - seq] : d.live.ab[seq - nf];
+    const int side = ab.x == g ? 0 : 1;
+    const int other = side == 0 ? ab.y : ab.x;
+    d.adjInfo[e] = (other >= 0 ? other : kNoBody) | static_cast<int>(static_cast<unsigned>(side) << 31);
+    if (seq >= nf)
+        reinterpret_cast<int *>(d.stampSlot)[2 * (seq - nf) + side] = e;
+}
+
 __global__ void adjInfoKernel(Dev d) {
     pdlWait();
     pdlTrigger();
@@ -81,16 +92,8 @@ __global__ void adjInfoKernel(Dev d) {
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= n)
         return;
-    const int nf = d.ctr[C_FORCES];
-    for (int e = d.adjStart[g]; e < d.adjStart[g + 1]; e++) {
-        const int seq = static_cast<int>(d.adjSeq[e]);
-        const int2 ab = seq < nf ? d.fAB[nf - 1 - seq] : d.live.ab[seq - nf];
-        const int side = ab.x == g ? 0 : 1;
-        const int other = side == 0 ? ab.y : ab.x;
-        d.adjInfo[e] = (other >= 0 ? other : kNoBody) | static_cast<int>(static_cast<unsigned>(side) << 31);
-        if (seq >= nf)
-            reinterpret_cast<int *>(d.stampSlot)[2 * (seq - nf) + side] = e;
-    }
+    for (int e = d.adjStart[g]; e < d.adjStart[g + 1]; e++)
+        adjInfoAt(d, g, e, static_cast<int>(d.adjSeq[e]));
 }
 
 __global__ void adjTotalKernel(Dev d) {
@@ -320,6 +323,40 @@ __global__ void manifoldInitKernel(Dev d, StepParams p) {
         manifoldInitAt<ROUND>(d, p, i);
 }
 
+// Contact slot c of candidate i (and, for slot 0, its record) to live manifold r.
+__device__ __forceinline__ void compactSlot(const Dev &d, int i, int c, int r) {
+    const ManifoldBuf &L = d.live, &S = d.stage;
+    const int n = S.count[i];
+    const int2 dorm = S.dormant[i];
+    if (c == 0) {
+        L.ab[r] = S.ab[i];
+        L.b0[r] = S.b0[i];
+        L.b1[r] = S.b1[i];
+        L.b2[r] = S.b2[i];
+        L.count[r] = n;
+        L.dormant[r] = dorm;
+        if (d.ARM) {
+            L.armFlag[r] = S.armFlag[i];
+            L.capA[r] = S.capA[i];
+            L.capB[r] = S.capB[i];
+        }
+    }
+    const int kept = n > 0 ? n : dorm.y; // a parked manifold keeps its saved contacts
+    if (c >= kept)
+        return;
+    const int si = cslot(d, i, c), di = cslot(d, r, c);
+    L.key[di] = S.key[si];
+    L.rA[di] = S.rA[si];
+    L.rB[di] = S.rB[si];
+    L.C0[di] = S.C0[si];
+    L.k[di] = S.k[si];
+    L.lam[di] = S.lam[si];
+    if (d.ARM) {
+        L.armA[di] = S.armA[si];
+        L.armB[di] = S.armB[si];
+    }
+}
+
 // One thread per contact slot (8 per candidate, slot-major like the arrays), so the copies of the
 // contact arrays coalesce; the slot-0 thread also moves the manifold's own record. Grid-stride.
 // Index type T: 32-bit where the slot count fits (the usual case; its division is far cheaper).
@@ -327,43 +364,13 @@ template <typename T>
 __device__ __forceinline__ void manifoldCompactRun(const Dev &d, const int *flags, const int *rank, int cand) {
     const T slots = static_cast<T>(cand) * kMaxContacts;
     const T stride = static_cast<T>(gridDim.x) * blockDim.x;
-    const ManifoldBuf L = d.live;
-    const ManifoldBuf S = d.stage;
     for (T t = static_cast<T>(blockIdx.x) * blockDim.x + threadIdx.x; t < slots; t += stride) {
         const int c = static_cast<int>(t / static_cast<T>(cand));
         const int i = static_cast<int>(t - static_cast<T>(c) * static_cast<T>(cand));
         if (!flags[i])
             continue;
         const int r = rank ? rank[i] : flags[i] - 1; // one world: its rank; several: its place
-        const int n = S.count[i];
-        const int2 dorm = S.dormant[i];
-        if (c == 0) {
-            L.ab[r] = S.ab[i];
-            L.b0[r] = S.b0[i];
-            L.b1[r] = S.b1[i];
-            L.b2[r] = S.b2[i];
-            L.count[r] = n;
-            L.dormant[r] = dorm;
-            if (d.ARM) {
-                L.armFlag[r] = S.armFlag[i];
-                L.capA[r] = S.capA[i];
-                L.capB[r] = S.capB[i];
-            }
-        }
-        const int kept = n > 0 ? n : dorm.y; // a parked manifold keeps its saved contacts
-        if (c >= kept)
-            continue;
-        const int si = cslot(d, i, c), di = cslot(d, r, c);
-        L.key[di] = S.key[si];
-        L.rA[di] = S.rA[si];
-        L.rB[di] = S.rB[si];
-        L.C0[di] = S.C0[si];
-        L.k[di] = S.k[si];
-        L.lam[di] = S.lam[si];
-        if (d.ARM) {
-            L.armA[di] = S.armA[si];
-            L.armB[di] = S.armB[si];
-        }
+        compactSlot(d, i, c, r);
     }
 }
 
@@ -377,6 +384,144 @@ __global__ void manifoldCompactKernel(Dev d, const int *flags, const int *rank) 
         manifoldCompactRun<unsigned>(d, flags, rank, cand);
     else
         manifoldCompactRun<unsigned long long>(d, flags, rank, cand);
+}
+
+// ---- one world's narrow phase, compaction, adjacency and update set in one launch ----
+//
+// What launchManifoldInit, launchManifoldCompact, launchAdjacency and, with `select` (no sleeping, no
+// greedy colouring), launchContactOnly and launchColourLists do, by one cluster: ~20 launches' fixed
+// costs for a store of one world of up to some thousand bodies.
+constexpr int kContactThreads = 512;
+
+template <bool ROUND>
+__global__ void __launch_bounds__(kContactThreads, 1)
+        worldContactsKernel(const __grid_constant__ Dev d, const __grid_constant__ StepParams p, int select) {
+    pdlWait();
+    pdlTrigger();
+    __shared__ int warpSums[kContactThreads / 32], ranks[kContactThreads], longCount;
+    const int rank = clusterRank(), size = clusterSize(), lane = threadIdx.x & 31;
+    // Threads over the cluster a warp at a time, so that few items still spread over its SMs.
+    const int tid = (size * static_cast<int>(threadIdx.x >> 5) + rank) * 32 + lane, threads = size * kContactThreads;
+    const int n = d.ctr[C_BODIES], cand = d.ctr[C_CAND], nf = d.ctr[C_FORCES];
+    int *counts = d.adjFill, *filled = d.solveFail; // scratch per body
+    for (int g = tid; g < n; g += threads)
+        counts[g] = filled[g] = 0;
+    if (rank == 0 && threadIdx.x <= kMaxColours)
+        d.colourCount[threadIdx.x] = 0;
+    for (int i = tid; i < cand; i += threads)
+        manifoldInitAt<ROUND>(d, p, i);
+    clusterSync(size);
+    // Survivors keep their order: this CTA's candidates, a tile at a time.
+    const Share kept = clusterShare(d.mActive, cand, rank, size, warpSums);
+    for (int tile = kept.lo, run = kept.before; tile < kept.hi; tile += kContactThreads) {
+        const int i = tile + static_cast<int>(threadIdx.x);
+        const bool on = i < kept.hi && d.mActive[i];
+        int all;
+        const int r = run + blockPrefix(on ? 1 : 0, warpSums, all);
+        ranks[threadIdx.x] = on ? r : -1;
+        run += all;
+        __syncthreads();
+        const int here = min(kContactThreads, kept.hi - tile);
+        for (int t = threadIdx.x; t < here * kMaxContacts; t += kContactThreads) {
+            const int c = t / here, k = t - c * here;
+            if (ranks[k] >= 0)
+                compactSlot(d, tile + k, c, ranks[k]);
+        }
+        if (on) {
+            const int2 ab = d.stage.ab[i];
+            if (d.x[ab.x].w > 0.0f)
+                atomicAdd(&counts[ab.x], 1);
+            if (d.x[ab.y].w > 0.0f)
+                atomicAdd(&counts[ab.y], 1);
+        }
+        __syncthreads();
+    }
+    for (int f = tid; f < nf; f += threads) {
+        const int2 ab = d.fAB[f];
+        if (ab.x >= 0 && d.x[ab.x].w > 0.0f)
+            atomicAdd(&counts[ab.x], 1);
+        if (ab.y >= 0 && d.x[ab.y].w > 0.0f)
+            atomicAdd(&counts[ab.y], 1);
+    }
+    clusterSync(size);
+    const Share entries = clusterShare(counts, n, rank, size, warpSums);
+    for (int tile = entries.lo, run = entries.before; tile < entries.hi; tile += kContactThreads) {
+        const int g = tile + static_cast<int>(threadIdx.x);
+        int all;
+        const int start = run + blockPrefix(g < entries.hi ? counts[g] : 0, warpSums, all);
+        if (g < entries.hi)
+            d.adjStart[g] = start;
+        run += all;
+    }
+    if (rank == 0 && threadIdx.x == 0) {
+        d.adjStart[n] = entries.total;
+        d.ctr[C_ADJ] = entries.total;
+        d.ctr[C_LIVE] = kept.total;
+        if (entries.total > 2 * (d.FF + d.MM))
+            atomicOr(&d.ctr[C_ERRORS], kErrAdjacency);
+    }
+    clusterSync(size);
+    const auto fill = [&](int g, int seq) {
+        if (g >= 0 && d.x[g].w > 0.0f)
+            d.adjSeq[d.adjStart[g] + atomicAdd(&filled[g], 1)] = static_cast<uint32_t>(seq);
+    };
+    for (int k = tid; k < nf + kept.total; k += threads) {
+        const int2 ab = k < nf ? d.fAB[k] : d.live.ab[k - nf];
+        const int seq = k < nf ? nf - 1 - k : k;
+        fill(ab.x, seq);
+        fill(ab.y, seq);
+    }
+    clusterSync(size);
+    // Each body's entries in sequence order; short runs by a thread, longer ones by the block.
+    if (threadIdx.x == 0)
+        longCount = 0;
+    __syncthreads();
+    int *longs = d.longList + entries.lo;
+    for (int g = entries.lo + static_cast<int>(threadIdx.x); g < entries.hi; g += kContactThreads) {
+        const int b = d.adjStart[g], e = d.adjStart[g + 1];
+        if (e - b > 32) {
+            longs[atomicAdd(&longCount, 1)] = g;
+            continue;
+        }
+        for (int i = b + 1; i < e; i++) {
+            const uint32_t x = d.adjSeq[i];
+            int j = i - 1;
+            for (; j >= b && d.adjSeq[j] > x; j--)
+                d.adjSeq[j + 1] = d.adjSeq[j];
+            d.adjSeq[j + 1] = x;
+        }
+        for (int i = b; i < e; i++)
+            adjInfoAt(d, g, i, static_cast<int>(d.adjSeq[i]));
+    }
+    __syncthreads();
+    for (int k = 0; k < longCount; k++) {
+        const int g = longs[k], b = d.adjStart[g], e = d.adjStart[g + 1];
+        for (int i = b + static_cast<int>(threadIdx.x); i < e; i += kContactThreads)
+            d.adjTmp[i] = d.adjSeq[i];
+        __syncthreads();
+        for (int i = b + static_cast<int>(threadIdx.x); i < e; i += kContactThreads) {
+            const uint32_t x = d.adjTmp[i];
+            int before = 0;
+            for (int j = b; j < e; j++)
+                before += d.adjTmp[j] < x ? 1 : 0;
+            d.adjSeq[b + before] = x;
+            adjInfoAt(d, g, b + before, static_cast<int>(x));
+        }
+        __syncthreads();
+    }
+    if (select) {
+        int updated = 0;
+        for (int g = entries.lo + static_cast<int>(threadIdx.x); g < entries.hi; g += kContactThreads) {
+            const bool dyn = d.x[g].w > 0.0f, update = selectBody(d, g, dyn);
+            d.contactOnly[g] = 1;
+            d.upd[g] = update ? 1 : 0;
+            d.colour[g] = update || !dyn ? kOverflowColour : kNotUpdated; // contact-only bodies overflow
+            updated += update ? 1 : 0;
+        }
+        updated = blockSum(updated, warpSums);
+        if (threadIdx.x == 0 && updated)
+            atomicAdd(&d.colourCount[kOverflowColour], updated);
+    }
 }
 
 // ---- world-major order ----
@@ -541,6 +686,28 @@ void launchAdjacency(const Dev &d, cudaStream_t s) {
 
 bool narrowBlockFits(int block) {
     return blockFits(manifoldInitKernel<false>, block) && blockFits(manifoldInitKernel<true>, block);
+}
+
+static int g_contactTeam = 0;
+
+static int contactTeamMax() {
+    if (g_contactTeam == 0) {
+        const int a = allowTeam(reinterpret_cast<const void *>(worldContactsKernel<false>), kContactThreads, 0);
+        const int b = allowTeam(reinterpret_cast<const void *>(worldContactsKernel<true>), kContactThreads, 0);
+        g_contactTeam = a < b ? a : b;
+    }
+    return g_contactTeam;
+}
+
+void prepareWorldContacts() { contactTeamMax(); }
+
+void launchWorldContacts(const Dev &d, const StepParams &p, bool round, bool select, int bodies, cudaStream_t s) {
+    int team = 1;
+    while (team < contactTeamMax() && team * 16 < bodies)
+        team *= 2;
+    const TeamLaunch l(team, 1, kContactThreads, 0, s);
+    ++launchCount();
+    cudaLaunchKernelEx(&l.cfg, round ? worldContactsKernel<true> : worldContactsKernel<false>, d, p, select ? 1 : 0);
 }
 
 void launchManifoldInit(const Dev &d, const StepParams &p, bool round, int block, cudaStream_t s) {

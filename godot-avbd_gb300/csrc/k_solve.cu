@@ -16,6 +16,7 @@
 #include "gridsync.cuh"
 #include "kernels.cuh"
 #include "prims.cuh"
+#include "project.cuh"
 #include "solve.cuh"
 
 namespace avbdg {
@@ -255,27 +256,11 @@ __global__ void finishKernel(Dev d, StepParams p, int idle) {
 __global__ void contactOnlyInitKernel(Dev d) {
     pdlWait();
     pdlTrigger();
-    const int n = d.ctr[C_BODIES];
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= n)
+    if (g >= d.ctr[C_BODIES])
         return;
+    const bool dyn = d.meta[g].x >= 0 && d.x[g].w > 0.0f, update = selectBody(d, g, dyn);
     d.contactOnly[g] = 1;
-    // The update set (solver_solve.cpp:296-339): movable bodies, minus idle sleepers (mode 1) and
-    // untouched, motionless bodies that start asleep (mode 2); a mode-2 sleeper otherwise wakes.
-    const bool dyn = d.meta[g].x >= 0 && d.x[g].w > 0.0f;
-    bool update = dyn;
-    if (dyn) {
-        const int mode = (d.meta[g].w >> 16) & 0x3;
-        const int2 s = d.sleep[g];
-        if (mode == 1) {
-            update = s.x == 0;
-        } else if (mode == 2) {
-            if (!s.x && length2(xyz(d.v[g])) == 0.0f && d.adjStart[g] == d.adjStart[g + 1])
-                update = false;
-            else if (s.x)
-                d.sleep[g] = make_int2(0, s.y);
-        }
-    }
     d.upd[g] = update ? 1 : 0;
     d.colour[g] = update ? kUncoloured : (dyn ? kNotUpdated : kOverflowColour);
 }
@@ -435,6 +420,8 @@ static int sweepGridMax() {
 
 void prepareKernels() {
     worldTeamMax();
+    worldPairsMost();
+    prepareWorldContacts();
     sweepGridMax();
     queueGridMax();
     projectionGridBlocks();

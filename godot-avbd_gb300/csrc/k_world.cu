@@ -28,6 +28,7 @@
 
 #include <algorithm>
 
+#include "cluster.cuh"
 #include "kernels.cuh"
 #include "prims.cuh"
 #include "project.cuh"
@@ -37,7 +38,6 @@ namespace avbdg {
 
 namespace {
 
-constexpr int kMaxTeam = 16;
 constexpr int kMaxWorldThreads = 512;
 constexpr int kWideThreads = 256;
 constexpr int kTaskManifolds = 8; // manifolds a task of 32 contact slots may hold: 96 groups of four sums
@@ -86,15 +86,6 @@ struct World {
     int mf, link, basis, cap, taskFirst;     // manifolds
     int slots, contacts;                     // contact slots
 };
-
-__device__ __forceinline__ void clusterSync(int size) {
-    if (size == 1) {
-        __syncthreads();
-    } else {
-        asm volatile("barrier.cluster.arrive.release;" ::: "memory");
-        asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
-    }
-}
 
 // Shared-memory addresses, of this CTA or (mapped) of another of the cluster.
 __device__ __forceinline__ unsigned sharedAddress(const void *p) { return static_cast<unsigned>(__cvta_generic_to_shared(p)); }
@@ -1336,11 +1327,8 @@ __global__ void __launch_bounds__(kMaxWorldThreads, 1)
     // it needs.
     __shared__ World w;
     if (threadIdx.x == 0) {
-        int rank, size;
-        asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
-        asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(size));
-        w.rank = rank;
-        w.size = size;
+        w.rank = clusterRank();
+        w.size = clusterSize();
     }
     __syncthreads();
     const int size = w.size, nWorlds = d.ctr[C_WORLDS];
@@ -1470,9 +1458,7 @@ __global__ void __launch_bounds__(kWideThreads)
     pdlWait();
     pdlTrigger();
     extern __shared__ __align__(32) unsigned char smem[];
-    int rank, size;
-    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
-    asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(size));
+    const int rank = clusterRank(), size = clusterSize();
     const int nWorlds = d.ctr[C_WORLDS];
     const int clusters = static_cast<int>(gridDim.x) / size;
     const int tid = rank * static_cast<int>(blockDim.x) + static_cast<int>(threadIdx.x), threads = size * static_cast<int>(blockDim.x);
@@ -1605,45 +1591,14 @@ constexpr int kSmemMost = 222 * 1024; // dynamic shared memory a CTA may have be
 
 int g_maxTeam = 0;
 
-// Cluster and (programmatic) stream attributes of a launch.
-struct TeamLaunch {
-    cudaLaunchConfig_t cfg{};
-    cudaLaunchAttribute attr[2]{};
-    TeamLaunch(int team, int worlds, int threads, size_t smem, cudaStream_t s) {
-        cfg.gridDim = dim3(static_cast<unsigned>(team) * static_cast<unsigned>(worlds));
-        cfg.blockDim = dim3(static_cast<unsigned>(threads));
-        cfg.dynamicSmemBytes = smem;
-        cfg.stream = s;
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = static_cast<unsigned>(team);
-        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[1].val.programmaticStreamSerializationAllowed = pdlEnabled() ? 1 : 0;
-        cfg.attrs = attr;
-        cfg.numAttrs = 2;
-    }
-};
-
 } // namespace
 
 int worldTeamMax() {
     if (g_maxTeam == 0) {
         int team = kMaxTeam;
         for (int c = 0; c < 4; c++) {
-            const void *k = reinterpret_cast<const void *>(worldKernelFor(c & 1, c & 2));
-            const void *wide = reinterpret_cast<const void *>(wideKernelFor(c & 1, c & 2));
-            cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMost);
-            cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-            cudaFuncSetAttribute(wide, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMost);
-            cudaFuncSetAttribute(wide, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-            for (; team > 1; team >>= 1) {
-                TeamLaunch l(team, 1, kMaxWorldThreads, kSmemMost, nullptr);
-                l.cfg.numAttrs = 1;
-                int n = 0;
-                if (cudaOccupancyMaxActiveClusters(&n, k, &l.cfg) == cudaSuccess && n > 0)
-                    break;
-                cudaGetLastError();
-            }
+            team = std::min(team, allowTeam(reinterpret_cast<const void *>(worldKernelFor(c & 1, c & 2)), kMaxWorldThreads, kSmemMost));
+            team = std::min(team, allowTeam(reinterpret_cast<const void *>(wideKernelFor(c & 1, c & 2)), kWideThreads, kSmemMost));
         }
         g_maxTeam = team;
     }

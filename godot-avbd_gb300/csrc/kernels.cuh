@@ -34,7 +34,16 @@ void launchPairs(const Dev &d, int block, bool brute, cudaStream_t s);
 // Exact filter and acquisition of new manifolds after the live ones (C_CAND = C_LIVE + new).
 void launchFilterAcquire(const Dev &d, cudaStream_t s);
 
+// One world's bounds, candidate pairs, filter and acquisition in one launch (launchAabb to
+// launchFilterAcquire without the tree): up to worldPairsMost() bodies.
+int worldPairsMost();
+void launchWorldPairs(const Dev &d, const StepParams &p, int bodies, cudaStream_t s);
+
 // ---- manifolds and adjacency (k_manifold.cu) ----
+// One world's narrow phase, compaction and adjacency in one launch, and with `select` (no sleeping, no
+// greedy colouring) its update set and colours.
+void prepareWorldContacts();
+void launchWorldContacts(const Dev &d, const StepParams &p, bool round, bool select, int bodies, cudaStream_t s);
 void launchAdjacency(const Dev &d, cudaStream_t s);
 void launchManifoldInit(const Dev &d, const StepParams &p, bool round, int block, cudaStream_t s);
 // `worldMajor`: survivors are ordered by world (each world's own order kept), world w's at

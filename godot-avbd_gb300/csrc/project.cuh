@@ -9,6 +9,25 @@ namespace avbdg {
 
 namespace {
 
+// Whether body g joins the step's update set (solver_solve.cpp:296-339): movable bodies (`dyn`), minus idle
+// sleepers (mode 1) and untouched, motionless bodies that start asleep (mode 2); a mode-2 sleeper
+// otherwise wakes here. Reads the adjacency of this step.
+__device__ __forceinline__ bool selectBody(const Dev &d, int g, bool dyn) {
+    if (!dyn)
+        return false;
+    const int mode = (d.meta[g].w >> 16) & 0x3;
+    const int2 s = d.sleep[g];
+    if (mode == 1)
+        return s.x == 0;
+    if (mode == 2) {
+        if (!s.x && length2(xyz(d.v[g])) == 0.0f && d.adjStart[g] == d.adjStart[g + 1])
+            return false;
+        if (s.x)
+            d.sleep[g] = make_int2(0, s.y);
+    }
+    return true;
+}
+
 // Movable and in this step's update set (solver_projection.cpp:87, 105-106, 194-195).
 __device__ __forceinline__ bool movable(const Dev &d, int g) { return d.x[g].w > 0.0f && inUpdate(d, g); }
 

@@ -91,3 +91,21 @@ def test_many_worlds_added_and_removed(pkg, gpu):
     for w in range(0, 50, 7):
         assert same([b.state(w)], [alone[w * 10 % 5][23]])
     assert same([b.state(50)], [alone[0][7]])
+
+
+# One wide dynamic plate (first or last in the store) under many small boxes: more adjacency entries than
+# a thread sorts, more partners of one body than the pair stash holds, and none.
+@pytest.mark.parametrize("boxes,last", [(20, False), (90, False), (90, True), (200, True)])
+def test_wide_plate(pkg, gpu, oracle, boxes, last):
+    capi = pkg.capi
+    rng = np.random.default_rng(boxes)
+    side = int(np.ceil(boxes ** 0.5))
+    i = np.arange(boxes)
+    pos = np.stack([0.6 * (i % side), 0.6 * (i // side), 1.0 + 0 * i], 1) + rng.uniform(-0.02, 0.02, (boxes, 3))
+    size, density = [[0.4, 0.4, 0.4]] * boxes, [1.0] * boxes
+    plate = [[0.6 * side + 2, 0.6 * side + 2, 0.3]], [5.0], [[0.3 * side, 0.3 * side, 0.45]]
+    ground = [[60, 60, 1]], [0.0], [[0, 0, -0.5]]
+    parts = [ground, (size, density, pos.tolist()), plate] if last else [ground, plate, (size, density, pos.tolist())]
+    d = capi.make_body_descs(*[sum((list(p[k]) for p in parts), []) for k in (0, 1)], 0.5,
+                             sum((list(p[2]) for p in parts), []))
+    assert same(run(gpu, capi, d, 25), run(oracle, capi, d, 25))
