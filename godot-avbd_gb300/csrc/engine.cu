@@ -902,10 +902,10 @@ Engine::StepPlan Engine::planStep(int mode, int substeps, int rounds) {
             sortLiveByWorld();
         liveByWorld = plan.worldMajor || worlds() <= 1; // (a single world's order is its own)
     }
-    if (worldAllowed && !plan.greedy && (plan.worldMajor || worlds() == 1)) {
+    if (worldAllowed && (plan.worldMajor || worlds() == 1)) {
         // Manifolds a body in the last checked step (a store's first step: a settled pile's).
         const double density = ctrFresh && nBodies > 0 ? static_cast<double>(hostCtr[C_LIVE]) / nBodies : 2.5;
-        if (worldsTake(count, bodies, density)) {
+        if (worldsTake(count, bodies, density, nBodies > 0 ? static_cast<double>(nForces) / nBodies : 0.0)) {
             plan.worldCount = count;
             plan.worldBodies = bodies;
         }

@@ -54,11 +54,9 @@ __device__ __forceinline__ f3 genericOffset(const Dev &d, int f) {
 
 // Angular measurement, swing-twist split (generic_joint.cpp:49-98): each non-locked axis takes its
 // twist 2 atan2(v.n, w) out of the deviation, the locked axes read the remaining swing.
-__device__ __forceinline__ void genericAngles(const Dev &d, int f, real out[3]) {
-    const int2 ab = d.fAB[f];
+__device__ __forceinline__ void genericAnglesOf(const Dev &d, int f, q4 qA, q4 qB, real out[3]) {
     const real4 *e = d.fExt + static_cast<size_t>(f) * kExtF4;
-    const q4 qA = frameOrientation(d, ab.x);
-    const q4 relativeNow = qmul(qconj(qA), qnormalize(asq(d.q[ab.y])));
+    const q4 relativeNow = qmul(qconj(qA), qnormalize(qB));
     q4 dev = qmul(qnormalize(asq(e[0])), qconj(relativeNow));
     int locked[3];
     for (int i = 0; i < 3; i++)
@@ -79,6 +77,11 @@ __device__ __forceinline__ void genericAngles(const Dev &d, int f, real out[3]) 
     for (int i = 0; i < 3; i++)
         if (locked[i])
             out[i] = qcomp(dev, i) * 2.0f;
+}
+
+__device__ __forceinline__ void genericAngles(const Dev &d, int f, real out[3]) {
+    const int2 ab = d.fAB[f];
+    genericAnglesOf(d, f, frameOrientation(d, ab.x), asq(d.q[ab.y]), out);
 }
 
 // axisConstraint + axisForce (generic_joint.cpp:120-168).
@@ -229,37 +232,52 @@ __device__ __forceinline__ void genericInit(const Dev &d, const StepParams &p, i
     e[14] = mk4(init[4], init[5], 0.0f, 0.0f);
 }
 
-// GenericJoint::updateDual (generic_joint.cpp:289-319).
+// GenericJoint::updateDual (generic_joint.cpp:289-319): axis `idx` (0-2 linear, 3-5 angular), measured
+// as `value`.
+__device__ __forceinline__ void genericDualValue(const Dev &d, const StepParams &p, int f, int idx, real value) {
+    const int2 ab = d.fAB[f];
+    const bool angular = idx >= 3;
+    real4 *e = d.fExt + static_cast<size_t>(f) * kExtF4;
+    const GAxis ax = loadAxis(d, f, idx);
+    real C, F;
+    real4 s = e[7 + idx];
+    if (!axisForce(ax, value, p.alpha, C, F)) {
+        if (ax.mode == kAxisLimited) {
+            s.z = 0.0f;
+            e[7 + idx] = s;
+        }
+        return;
+    }
+    s.z = F;
+    const f3 dir = qrot(frameOrientation(d, ab.x), unitAxis(angular ? idx - 3 : idx));
+    real cap = penaltyLimit(d, p, ab.y, dir, angular);
+    if (ab.x >= 0)
+        cap = smin(cap, penaltyLimit(d, p, ab.x, dir, angular));
+    s.w = sclamp(ax.penalty + mabs(C) * (angular ? p.betaAng : p.betaLin), 0.0f, cap);
+    e[7 + idx] = s;
+}
+
 __device__ __forceinline__ void genericDual(const Dev &d, const StepParams &p, int f) {
     real ang[3];
     genericAngles(d, f, ang);
     const f3 offset = genericOffset(d, f);
-    const int2 ab = d.fAB[f];
-    real4 *e = d.fExt + static_cast<size_t>(f) * kExtF4;
     for (int i = 0; i < 3; i++) {
-        const real values[2] = {at(offset, i), ang[i]};
-        const real betas[2] = {p.betaLin, p.betaAng};
-        for (int k = 0; k < 2; k++) {
-            const int idx = 3 * k + i;
-            const GAxis ax = loadAxis(d, f, idx);
-            real C, F;
-            real4 s = e[7 + idx];
-            if (!axisForce(ax, values[k], p.alpha, C, F)) {
-                if (ax.mode == kAxisLimited) {
-                    s.z = 0.0f;
-                    e[7 + idx] = s;
-                }
-                continue;
-            }
-            s.z = F;
-            const f3 dir = qrot(frameOrientation(d, ab.x), unitAxis(i));
-            real cap = penaltyLimit(d, p, ab.y, dir, k == 1);
-            if (ab.x >= 0)
-                cap = smin(cap, penaltyLimit(d, p, ab.x, dir, k == 1));
-            s.w = sclamp(ax.penalty + mabs(C) * betas[k], 0.0f, cap);
-            e[7 + idx] = s;
-        }
+        genericDualValue(d, p, f, i, at(offset, i));
+        genericDualValue(d, p, f, 3 + i, ang[i]);
     }
+}
+
+// One axis alone (its measurement does not depend on the others' forces).
+__device__ __forceinline__ void genericDualAxis(const Dev &d, const StepParams &p, int f, int idx) {
+    real value;
+    if (idx < 3) {
+        value = at(genericOffset(d, f), idx);
+    } else {
+        real ang[3];
+        genericAngles(d, f, ang);
+        value = idx == 3 ? ang[0] : (idx == 4 ? ang[1] : ang[2]);
+    }
+    genericDualValue(d, p, f, idx, value);
 }
 
 } // namespace avbdg

@@ -17,6 +17,9 @@
 //             from zero.
 //   bodies    the block's thirty sums are one lane each: a warp adds a body's stamp records in entry
 //             order; a thread per body then factorises.
+//   colours   the coloured bodies are dealt round the CTAs, wherever their state lies. A lane takes a
+//             contact of one's manifolds or a part of one of its forces, lanes of a kind together in a
+//             warp; a warp a body then adds the terms in adjacency order.
 //   brake     a single CTA of the cluster runs the sweep, level by level of its dependencies, with the
 //             world's velocities in shared memory.
 //
@@ -68,8 +71,8 @@ __device__ __forceinline__ bool mfActive(int f) { return (f & (kMfMoveA | kMfMov
 enum : int { kRecAng = 3, kRecX = 4, kRecQ = 5, kRecMoment = 6, kRecF4 = 7 };
 // Its step constants: inertial position and orientation, step-start position and orientation.
 enum : int { kConXi = 0, kConQi = 1, kConX0 = 2, kConQ0 = 3, kConF4 = 4 };
-// Body flags: colour, in the update set, movable, axis locks.
-enum : int { kBiColour = 0xf, kBiUpdate = 16, kBiMovable = 32, kBiLocks = 8 };
+// Body flags: colour, in the update set, movable, has a force, axis locks.
+enum : int { kBiColour = 0xf, kBiUpdate = 16, kBiMovable = 32, kBiForce = 64, kBiLocks = 8 };
 
 // The world a cluster works on and this CTA's part of it, with the byte offsets of its arrays.
 struct World {
@@ -85,6 +88,11 @@ struct World {
     int sums, info, entry, rec, con, stamps; // bodies
     int mf, link, basis, cap, taskFirst;     // manifolds
     int slots, contacts;                     // contact slots
+    // The coloured bodies dealt to this CTA, by colour, their blocks and their terms.
+    int colourList, colourBlocks, termFirst, terms, termOrder, termKinds;
+    int colourAt[kMaxColours + 1]; // first of each colour in the list
+    int groupAt[kMaxColours + 1];  // first group of terms of each colour
+    int rec0, con0;                // this CTA's address of the pose records and step constants
 };
 
 // Shared-memory addresses, of this CTA or (mapped) of another of the cluster.
@@ -384,30 +392,60 @@ __device__ __forceinline__ void movePose(const Dev &d, const World &w, unsigned 
     }
 }
 
-// The blocks before their manifolds (makeBlock; with COLOURS the forces, which come first in an
-// adjacency): while a round's contact tasks run, the body warps already prepare the next round's.
+// Where the records of a body of the world (counted from its first) lie.
+struct BodyPlace {
+    unsigned rec, con;
+};
+__device__ __forceinline__ BodyPlace placeOf(const World &w, int i) {
+    const int o = i / w.per, k = i - o * w.per;
+    return BodyPlace{mapShared(w.rec0, o) + kF4 * kRecF4 * k, mapShared(w.con0, o) + kF4 * kConF4 * k};
+}
+
+// The blocks of the bodies to solve before their forces and manifolds (makeBlock, from the body's own
+// pose): while a round's contact tasks run, the body warps already prepare the next round's.
 template <bool COLOURS>
-__device__ __forceinline__ void startBlocks(const Dev &d, const StepParams &p, const World &w, unsigned char *smem) {
-    const int *info = arrayAt<int>(smem, w.info), *entry = arrayAt<int>(smem, w.entry);
-    real *sums = arrayAt<real>(smem, w.sums);
-    const int nb = w.nb;
-    for (int i = bodyThread(); i < nb; i += blockDim.x) {
+__device__ __forceinline__ void startBlocks(const StepParams &p, const World &w, unsigned char *smem) {
+    const int *info = arrayAt<int>(smem, w.info);
+    const int nb = w.nb, coloured = COLOURS ? w.colourAt[kMaxColours] : 0;
+    for (int k = bodyThread(); k < nb + coloured; k += blockDim.x) {
+        if (COLOURS && k < coloured) {
+            const BodyPlace at = placeOf(w, arrayAt<uint16_t>(smem, w.colourList)[k]);
+            const real4 x4 = loadCluster(at.rec + kRecX * kF4);
+            putBlock(arrayAt<real>(smem, w.colourBlocks) + k * kBlkReals,
+                     makeBlock(x4.w, xyz(loadCluster(at.rec + kRecMoment * kF4)), p.dtSq, xyz(x4),
+                               xyz(loadCluster(at.con + kConXi * kF4)), asq(loadCluster(at.rec + kRecQ * kF4)),
+                               asq(loadCluster(at.con + kConQi * kF4))));
+            continue;
+        }
+        const int i = k - coloured;
         if (!overflowBody(info[i]))
             continue;
         const real4 *r = arrayAt<real4>(smem, w.rec) + kRecF4 * i, *con = arrayAt<real4>(smem, w.con) + kConF4 * i;
         const real4 x4 = r[kRecX];
-        Blk blk = makeBlock(x4.w, xyz(r[kRecMoment]), p.dtSq, xyz(x4), xyz(con[kConXi]), asq(r[kRecQ]), asq(con[kConQi]));
-        if (COLOURS) {
-            const int nf = nForcesDev(d);
-            for (int e = entry[i]; e < entry[i + 1]; e++) {
-                const int seq = static_cast<int>(d.adjSeq[e]);
-                if (seq >= nf)
-                    break;
-                jointStamp(d, p, nf - 1 - seq, w.b0 + i, blk);
-            }
-        }
-        putBlock(sums + i * kBlkReals, blk);
+        putBlock(arrayAt<real>(smem, w.sums) + i * kBlkReals,
+                 makeBlock(x4.w, xyz(r[kRecMoment]), p.dtSq, xyz(x4), xyz(con[kConXi]), asq(r[kRecQ]), asq(con[kConQi])));
     }
+}
+
+// The forces of overflow bodies (they come first in an adjacency) onto their blocks: bodies past the
+// last colour are rare.
+__device__ __forceinline__ void overflowForces(const Dev &d, const StepParams &p, const World &w, unsigned char *smem) {
+    const int *info = arrayAt<int>(smem, w.info), *entry = arrayAt<int>(smem, w.entry);
+    const int nf = nForcesDev(d);
+    for (int i = threadIdx.x; i < w.nb; i += blockDim.x) {
+        if (!overflowBody(info[i]) || !(info[i] & kBiForce))
+            continue;
+        real *sum = arrayAt<real>(smem, w.sums) + i * kBlkReals;
+        Blk blk = getBlock(sum);
+        for (int e = entry[i]; e < entry[i + 1]; e++) {
+            const int seq = static_cast<int>(d.adjSeq[e]);
+            if (seq >= nf)
+                break;
+            jointStamp(d, p, nf - 1 - seq, w.b0 + i, blk);
+        }
+        putBlock(sum, blk);
+    }
+    __syncthreads();
 }
 
 // Overflow bodies of this CTA: add the stamp records, factorise, apply (solveAt). Bodies with a force
@@ -426,9 +464,9 @@ __device__ __forceinline__ void solvePhase(const Dev &d, const StepParams &p, co
                 continue;
             int e = entry[i] - e0;
             const int e1 = entry[i + 1] - e0;
-            if (COLOURS) {
+            if (COLOURS && (info[i] & kBiForce)) {
                 const int nf = nForcesDev(d);
-                while (nf > 0 && e < e1 && static_cast<int>(d.adjSeq[e0 + e]) < nf)
+                while (e < e1 && static_cast<int>(d.adjSeq[e0 + e]) < nf)
                     e++;
             }
             real v = sums[i * kBlkReals + lane];
@@ -452,13 +490,11 @@ __device__ __forceinline__ void solvePhase(const Dev &d, const StepParams &p, co
             dl = r.ok ? r.dl : f3{0, 0, 0};
             da = r.ok ? r.da : f3{0, 0, 0};
         }
-        if (COLOURS) {
+        if (COLOURS && (info[i] & kBiForce)) {
             const int g = w.b0 + i;
-            if (bodyHasForce(d, g, nForcesDev(d))) {
-                d.dLin[g] = f4(dl, 0.0f);
-                d.dAng[g] = f4(da, 0.0f);
-                continue;
-            }
+            d.dLin[g] = f4(dl, 0.0f);
+            d.dAng[g] = f4(da, 0.0f);
+            continue;
         }
         const real4 *r = arrayAt<real4>(smem, w.rec) + kRecF4 * i;
         const real4 x4 = r[kRecX];
@@ -470,7 +506,8 @@ __device__ __forceinline__ void solvePhase(const Dev &d, const StepParams &p, co
 __device__ __forceinline__ void applyPhase(const Dev &d, const StepParams &p, const World &w, unsigned char *smem) {
     for (int i = threadIdx.x; i < w.nb; i += blockDim.x) {
         const int g = w.b0 + i;
-        if (!overflowBody(arrayAt<int>(smem, w.info)[i]) || !bodyHasForce(d, g, nForcesDev(d)))
+        const int info = arrayAt<int>(smem, w.info)[i];
+        if (!overflowBody(info) || !(info & kBiForce))
             continue;
         const real4 *r = arrayAt<real4>(smem, w.rec) + kRecF4 * i;
         const real4 x4 = r[kRecX];
@@ -479,23 +516,392 @@ __device__ __forceinline__ void applyPhase(const Dev &d, const StepParams &p, co
     }
 }
 
-// One round's Gauss-Seidel colours in order, a barrier after each.
+// ---- colours (solver_step.cpp:209-229) ----
+//
+// A coloured body's block is its start (startBlocks), then its forces' terms, then its manifolds', in
+// adjacency order. Each is a list of terms fixed for the step: a force's parts (a ball joint's linear
+// stamp, its geometric stiffness and its angular stamp; a spring; a generic joint's constraint and spring
+// of each axis that has them) and a manifold side's contacts (the same terms recomputeSide adds). A
+// term is a lane's work and leaves its thirty values in a row of shared memory, in order; thirty lanes
+// then add the rows, a manifold's contacts summed from zero first. A colour is a chain of one body's
+// latencies (poses over the cluster, a term's code, the sum, the factorisation), so its terms are sorted by
+// kind, a warp to a kind, and its bodies are dealt round the CTAs (ragdolls lie side by side in a store).
+// A level of 600 bodies with 114 coloured ones took 92 us a round in the separate sweep; 27k cycles (13 us)
+// a colour with each body at its owner and one warp taking its kinds in turn; 16k this way, of which the
+// terms take half and the factorisation a fifth.
+
+// Kinds of terms.
+enum : int { kTermContact, kTermBallLinear, kTermBallGeometric, kTermBallAngular, kTermSpring, kTermLinear, kTermAngular, kTermKinds };
+// A term: its kind, force (or contact and manifold), and the records of its bodies A and B (0: none).
+struct __align__(16) Term {
+    int flags, id;
+    unsigned recA, recB;
+    int manifold, row; // row: its place in the world's list of this CTA
+};
+enum : int {
+    kTermKind = 0xf,
+    kTermFirst = 16, kTermLast = 32, // of a manifold's contacts
+    kTermSideB = 64,                 // the body is B
+    kTermDualArms = 128,             // arm cache: after a dual, the first touch takes the arms it left
+    kTermPart = 8                    // (shift) a generic joint's axis 0-2, + 4 for its spring
+};
+constexpr int kRowMark = 51; // place of the flags in a row
+
+struct TermPose {
+    f3 x;
+    q4 q;
+};
+__device__ __forceinline__ TermPose termPose(unsigned rec) {
+    if (!rec)
+        return TermPose{f3{0, 0, 0}, q4{0.0f, 0.0f, 0.0f, 1.0f}};
+    return TermPose{xyz(loadCluster(rec + kRecX * kF4)), asq(loadCluster(rec + kRecQ * kF4))};
+}
+
+// ballStamp's parts (joint.cpp:80-175).
+// What a part does not touch stays -0, which no sum feels.
+__device__ __forceinline__ void ballPart(const Dev &d, const StepParams &p, int f, int kind, bool isA, const Term &t, Blk &k) {
+    const real4 par = d.fPar[f];
+    const TermPose A = termPose(t.recA), B = termPose(t.recB);
+    if (kind == kTermBallAngular) {
+        const f3 ka = xyz(d.fKA[f]);
+        if (!(length2(ka) > 0))
+            return;
+        const m3 K = mdiag(ka.x, ka.y, ka.z);
+        f3 C = scale(qdiff(A.q, B.q), par.w);
+        if (isinf(par.y))
+            C = sub(C, scale(xyz(d.fC0A[f]), p.alpha));
+        const f3 F = add(mul(K, C), xyz(d.fLA[f]));
+        const m3 base = isA ? mdiag(1, 1, 1) : mcols(f3{0, 0, 0}, f3{0, -1, 0}, f3{0, 0, -1});
+        const m3 jAng = mscale(base, par.w);
+        k.ang = mul(mul(transpose(jAng), K), jAng);
+        k.ra = mul(transpose(jAng), F);
+        return;
+    }
+    const f3 kl = xyz(d.fKL[f]);
+    if (!(length2(kl) > 0))
+        return;
+    const m3 K = mdiag(kl.x, kl.y, kl.z);
+    const f3 rA = xyz(d.fRA[f]), rB = xyz(d.fRB[f]);
+    const f3 rotA = qrot(A.q, rA), rotB = qrot(B.q, rB);
+    f3 C = sub(t.recA ? add(A.x, rotA) : rA, add(B.x, rotB));
+    if (isinf(par.x))
+        C = sub(C, scale(xyz(d.fC0L[f]), p.alpha));
+    const f3 F = add(mul(K, C), xyz(d.fLL[f]));
+    if (kind == kTermBallGeometric) {
+        const f3 rr = isA ? rotA : neg(rotB);
+        const m3 H = madd(madd(mscale(geometricStiffness(0, rr), F.x), mscale(geometricStiffness(1, rr), F.y)),
+                          mscale(geometricStiffness(2, rr), F.z));
+        k.ang = mdiag(H.c0.x, H.c1.y, H.c2.z);
+        return;
+    }
+    const m3 I = mdiag(1, 1, 1);
+    const m3 jLin = isA ? I : mneg(I);
+    const f3 r = isA ? neg(rotA) : rotB;
+    const m3 jAng = mcols(f3{0, r.z, -r.y}, f3{-r.z, 0, r.x}, f3{r.y, -r.x, 0});
+    const m3 jLinT = transpose(jLin);
+    const m3 jAngT = transpose(jAng);
+    const m3 jAngTk = mul(jAngT, K);
+    k.lin = mul(mul(jLinT, K), jLin);
+    k.ang = mul(jAngTk, jAng);
+    k.crs = mul(jAngTk, jLin);
+    k.rl = mul(jLinT, F);
+    k.ra = mul(jAngT, F);
+}
+
+// springStamp (spring.cpp:31-70).
+__device__ __forceinline__ void springPart(const Dev &d, int f, bool isA, const Term &t, Blk &k) {
+    const real4 par = d.fPar[f];
+    const TermPose A = termPose(t.recA), B = termPose(t.recB);
+    const f3 rA = qrot(A.q, xyz(d.fRA[f])), rB = qrot(B.q, xyz(d.fRB[f]));
+    const f3 dv = sub(add(A.x, rA), add(B.x, rB));
+    const real len = length(dv);
+    if (len <= 1.0e-6f)
+        return;
+    const f3 n = divs(dv, len);
+    const real C = len - par.y;
+    const real force = par.x * C;
+    const f3 jLin = isA ? n : neg(n);
+    const f3 jAng = isA ? cross(rA, n) : neg(cross(rB, n));
+    k.lin = mscale(outerprod(jLin, jLin), par.x);
+    k.ang = mscale(outerprod(jAng, jAng), par.x);
+    k.crs = mscale(outerprod(jAng, jLin), par.x);
+    k.rl = scale(jLin, force);
+    k.ra = scale(jAng, force);
+}
+
+// One axis' constraint or spring of a generic joint (genericStamp, stampAxis).
+template <bool angular>
+__device__ __forceinline__ void genericPart(const Dev &d, const StepParams &p, int f, int part, bool isA, const Term &t, Blk &k) {
+    const int i = part & 3;
+    const bool spring = (part & 4) != 0;
+    const int2 ab = d.fAB[f];
+    const TermPose A = termPose(t.recA), B = termPose(t.recB);
+    const real sign = isA ? 1.0f : -1.0f;
+    const f3 rA = xyz(d.fRA[f]), rAWorld = qrot(A.q, rA), rBWorld = qrot(B.q, xyz(d.fRB[f]));
+    const f3 axis = qrot(A.q, unitAxis(i));
+    const GAxis ax = loadAxis(d, f, angular ? 3 + i : i);
+    f3 jLin{0, 0, 0}, jAng;
+    real value;
+    if (angular) {
+        real ang[3];
+        genericAnglesOf(d, f, A.q, B.q, ang);
+        value = i == 0 ? ang[0] : (i == 1 ? ang[1] : ang[2]);
+        jAng = scale(axis, sign);
+    } else {
+        const f3 anchorA = t.recA ? add(A.x, rAWorld) : rA;
+        value = at(qrot(qconj(A.q), sub(anchorA, add(B.x, rBWorld))), i);
+        jLin = scale(axis, sign);
+        jAng = cross(isA ? rAWorld : rBWorld, jLin);
+    }
+    real stiffness, F;
+    if (spring) {
+        const f3 wA = ab.x >= 0 ? xyz(d.w[ab.x]) : f3{0, 0, 0}, wB = xyz(d.w[ab.y]);
+        real rate;
+        if (angular) {
+            rate = dot(sub(wA, wB), axis);
+        } else {
+            const f3 vA = ab.x >= 0 ? add(xyz(d.v[ab.x]), cross(wA, rAWorld)) : f3{0, 0, 0};
+            const f3 vB = add(xyz(d.v[ab.y]), cross(wB, rBWorld));
+            rate = dot(sub(vA, vB), axis);
+        }
+        const real Cs = value - ax.springEq;
+        F = ax.springK * Cs - ax.springDamp * rate;
+        stiffness = ax.springK;
+    } else {
+        real C;
+        if (!axisForce(ax, value, p.alpha, C, F))
+            return;
+        stiffness = ax.penalty;
+    }
+    k.lin = mscale(outerprod(jLin, jLin), stiffness);
+    k.ang = mscale(outerprod(jAng, jAng), stiffness);
+    k.crs = mscale(outerprod(jAng, jLin), stiffness);
+    k.rl = scale(jLin, F);
+    k.ra = scale(jAng, F);
+}
+
+// A contact's terms of one side at the current poses (recomputeSide): its 27 values in record order.
+template <bool ARM>
+__device__ __forceinline__ void contactTerm(const Dev &d, const StepParams &p, const Term &t, int armsFromDual, real4 *row) {
+    const ManifoldBuf &L = d.live;
+    const int m = t.manifold, ci = t.id;
+    const real4 rA4 = L.rA[ci], rB4 = L.rB[ci], b04 = L.b0[m];
+    const f3 r0 = xyz(b04), r1 = xyz(L.b1[m]), r2 = xyz(L.b2[m]), C0 = xyz(L.C0[ci]), k = xyz(L.k[ci]), lam = xyz(L.lam[ci]);
+    const PoseRec A = readPose(t.recA), B = readPose(t.recB);
+    f3 rAw, rBw;
+    if (ARM && armsFromDual && (t.flags & kTermDualArms)) {
+        rAw = xyz(L.armA[ci]);
+        rBw = xyz(L.armB[ci]);
+    } else {
+        rAw = mul(A.rot, xyz(rA4));
+        rBw = mul(B.rot, xyz(rB4));
+        if (ARM) {
+            L.armA[ci] = f4(rAw, 0.0f);
+            L.armB[ci] = f4(rBw, 0.0f);
+        }
+    }
+    const f3 bracket = sub(add(sub(A.dLin, B.dLin), cross(A.dAng, rAw)), cross(B.dAng, rBw));
+    const f3 C = contactError(p, C0, bracket, r0, r1, r2);
+    f3 F = add(cmul(k, C), lam);
+    clampForce(F, b04.w);
+    real S[6];
+    basisHessianD(r0, r1, r2, k, S);
+    const f3 fw = add(add(scale(r0, F.x), scale(r1, F.y)), scale(r2, F.z));
+    row[0] = mk4(S[0], S[1], S[2], S[3]);
+    row[1] = mk4(S[4], S[5], fw.x, fw.y);
+    const SideTerms side = sideTerms(S, t.flags & kTermSideB ? rBw : rAw, fw);
+    putSide(row + 2, side, fw.z);
+    real *r = reinterpret_cast<real *>(row);
+    r[27] = side.h[1]; // the angular block's mirrored entries
+    r[28] = side.h[2];
+    r[29] = side.h[4];
+}
+
+// The rows a pass holds: a colour's terms in the CTA are taken in groups of this many.
+__device__ __forceinline__ int passRows() { return 32 * contactWarps(); }
+
+template <bool ARM>
 __device__ __forceinline__ void colourPhase(const Dev &d, const StepParams &p, const World &w, unsigned char *smem, int colours,
-                                            int armsFromDual) {
-    const int *info = arrayAt<int>(smem, w.info);
+                                            int armsFromDual, real *carry) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5, group = passRows();
+    real *rows = arrayAt<real>(smem, 0);
+    const int *termFirst = arrayAt<int>(smem, w.termFirst);
+    const Term *terms = arrayAt<Term>(smem, w.terms);
+    const uint16_t *order = arrayAt<uint16_t>(smem, w.termOrder);
+    const bool rhs = (lane >= 6 && lane < 9) || (lane >= 15 && lane < 18);
     for (int c = 0; c < kMaxColours; c++) {
         if (!((colours >> c) & 1))
             continue;
-        for (int i = threadIdx.x; i < w.nb; i += blockDim.x) {
-            if ((info[i] & (kBiUpdate | kBiColour)) != (kBiUpdate | c))
-                continue;
-            const int g = w.b0 + i;
-            colourBodyAt(d, p, g, armsFromDual);
-            const real4 x4 = d.x[g];
-            movePose(d, w, smem, i, xyz(x4), x4.w, asq(d.q[g]), false);
+        const int k0 = w.colourAt[c], k1 = w.colourAt[c + 1];
+        const int first = k0 < k1 ? termFirst[k0] : 0, last = k0 < k1 ? termFirst[k1] : 0;
+        for (int from = first, pass = 0; k0 < k1 && (pass == 0 || from < last); from += group, pass++) {
+            const int to = min(from + group, last);
+            // Terms: warps take up to 32 of a kind.
+            const uint16_t *kinds = arrayAt<uint16_t>(smem, w.termKinds) + (w.groupAt[c] + pass) * (kTermKinds + 1);
+            for (int task = warp, kind = 0, before = 0; kind < kTermKinds; kind++) {
+                const int a = kinds[kind], n = kinds[kind + 1] - a, tasks = (n + 31) >> 5;
+                for (; task < before + tasks; task += warps) {
+                    const int at = 32 * (task - before) + lane;
+                    if (at >= n)
+                        continue;
+                    const Term t = terms[order[from + a + at]];
+                    real *row = rows + (t.row - from) * kRowReals;
+                    const bool isA = !(t.flags & kTermSideB);
+                    if (kind == kTermContact) {
+                        contactTerm<ARM>(d, p, t, armsFromDual, reinterpret_cast<real4 *>(row));
+                    } else {
+                        Blk b;
+                        const f3 none{-0.0f, -0.0f, -0.0f};
+                        b.lin = b.ang = b.crs = mcols(none, none, none);
+                        b.rl = b.ra = none;
+                        if (kind == kTermSpring)
+                            springPart(d, t.id, isA, t, b);
+                        else if (kind == kTermLinear)
+                            genericPart<false>(d, p, t.id, t.flags >> kTermPart, isA, t, b);
+                        else if (kind == kTermAngular)
+                            genericPart<true>(d, p, t.id, t.flags >> kTermPart, isA, t, b);
+                        else
+                            ballPart(d, p, t.id, kind, isA, t, b);
+                        putBlock(row, b);
+                    }
+                    *reinterpret_cast<int *>(row + kRowMark) = t.flags;
+                }
+                before += tasks;
+            }
+            __syncthreads();
+            // Sums, a warp a body; a body whose terms go on in the next group leaves its sums for it.
+            for (int k = k0 + warp; k < k1; k += warps) {
+                const int t0 = termFirst[k], t1 = termFirst[k + 1];
+                const bool done = t1 <= from + group && (t1 > from || pass == 0);
+                if (!done && !(t0 < to && t1 > from))
+                    continue;
+                real *sums = arrayAt<real>(smem, w.colourBlocks) + k * kBlkReals;
+                real v = lane < 30 ? sums[lane] : 0.0f, acc = t0 < from ? carry[lane] : 0.0f;
+                const real *r = rows + (max(t0, from) - from) * kRowReals, *end = rows + (min(t1, to) - from) * kRowReals;
+#pragma unroll 4
+                for (; r < end; r += kRowReals) {
+                    const int mark = *reinterpret_cast<const int *>(r + kRowMark);
+                    // A force's term alone (-0 + x is x), a manifold's contacts from zero.
+                    acc = (mark & kTermFirst ? (mark & kTermKind ? -0.0f : 0.0f) : acc) + r[lane];
+                    const real next = v + (rhs && (mark & (kTermKind | kTermSideB)) == kTermSideB ? -acc : acc);
+                    v = mark & kTermLast ? next : v;
+                }
+                if (lane < 30)
+                    sums[lane] = v;
+                if (!done) {
+                    carry[lane] = acc;
+                    continue;
+                }
+                __syncwarp();
+                if (lane == 0) {
+                    const int i = arrayAt<uint16_t>(smem, w.colourList)[k];
+                    const BodyPlace at = placeOf(w, i);
+                    const real4 x4 = loadCluster(at.rec + kRecX * kF4), q4v = loadCluster(at.rec + kRecQ * kF4);
+                    const real4 x0 = loadCluster(at.con + kConX0 * kF4), q0 = loadCluster(at.con + kConQ0 * kF4);
+                    f3 dl, da;
+                    if (!solveBlockFast(getBlock(sums), dl, da)) {
+                        const Delta s = solveSlow(getBlock(sums));
+                        dl = s.ok ? s.dl : f3{0, 0, 0};
+                        da = s.ok ? s.da : f3{0, 0, 0};
+                    }
+                    const f3 x = add(xyz(x4), dl);
+                    const q4 q = qintegrate(asq(q4v), da);
+                    real4 rec[kRecMoment];
+                    putPose(rec, x, x4.w, q, xyz(x0), asq(q0));
+#pragma unroll
+                    for (int j = 0; j < kRecMoment; j++)
+                        storeCluster(at.rec + j * kF4, rec[j]);
+                    d.x[w.base + i] = rec[kRecX];
+                    d.q[w.base + i] = rec[kRecQ];
+                }
+            }
+            if (to < last)
+                __syncthreads();
         }
         clusterSync(w.size);
     }
+}
+
+// A force's dual pass by eight lanes: a generic joint's axes one each, any other force by the first. The
+// CTAs' last body warps take four forces each first: the first ones start the next round's blocks.
+__device__ __forceinline__ void forceDuals(const Dev &d, const StepParams &p, const World &w) {
+    const int last = static_cast<int>(blockDim.x >> 7) - 1 - static_cast<int>(threadIdx.x >> 7), axis = threadIdx.x & 7;
+    const int first = w.f0 + 4 * (w.rank + w.size * last) + (static_cast<int>(threadIdx.x & 31) >> 3);
+    for (int f = first; f < w.f1; f += 4 * w.size * static_cast<int>(blockDim.x >> 7)) {
+        if (d.fKind[f] == kForceGeneric) {
+            if (axis < 6)
+                genericDualAxis(d, p, f, axis);
+        } else if (axis == 0) {
+            forceDualAt(d, p, f);
+        }
+    }
+}
+
+// The terms of an adjacency entry of coloured body `g`, counted and given to `put`.
+template <typename RecOf, typename Put>
+__device__ __forceinline__ int entryTerms(const Dev &d, int g, int e, RecOf recOf, Put put) {
+    const int nf = nForcesDev(d), seq = static_cast<int>(d.adjSeq[e]), v = d.adjInfo[e], o = adjInfoOther(v), side = adjInfoSide(v);
+    const unsigned own = recOf(g), other = o >= 0 ? recOf(o) : 0;
+    Term t{side ? kTermSideB : 0, 0, side ? other : own, side ? own : other, 0, 0};
+    int n = 0;
+    const auto add = [&](int flags) {
+        Term a = t;
+        a.flags |= flags;
+        put(n++, a);
+    };
+    if (seq >= nf) {
+        t.manifold = seq - nf;
+        const int count = d.live.count[t.manifold];
+        if (!(o >= 0 && inUpdate(d, o) && d.colour[o] < d.colour[g]))
+            t.flags |= kTermDualArms;
+        for (int c = 0; c < count; c++) {
+            t.id = cslot(d, t.manifold, c);
+            add(kTermContact | (c == 0 ? kTermFirst : 0) | (c + 1 == count ? kTermLast : 0));
+        }
+        return n;
+    }
+    t.id = nf - 1 - seq;
+    t.flags |= kTermFirst | kTermLast;
+    const int kind = d.fKind[t.id];
+    if (kind == kForceBall) {
+        add(kTermBallLinear);
+        add(kTermBallGeometric);
+        add(kTermBallAngular);
+    } else if (kind == kForceSpring) {
+        add(kTermSpring);
+    } else if (kind == kForceGeneric) {
+        for (int i = 0; i < 6; i++) { // axis i / 2, linear then angular
+            const GAxis ax = loadAxis(d, t.id, (i >> 1) + 3 * (i & 1));
+            const int flags = (i & 1 ? kTermAngular : kTermLinear) | (i >> 1) << kTermPart;
+            if (ax.mode == kAxisLocked || ax.mode == kAxisLimited)
+                add(flags);
+            if (ax.springK > 0.0f)
+                add(flags | 4 << kTermPart);
+        }
+    }
+    return n;
+}
+
+// A body's entries by a warp: `put(n, term)` numbers its terms in order; their count.
+template <typename RecOf, typename Put>
+__device__ __forceinline__ int bodyTerms(const Dev &d, int g, RecOf recOf, Put put) {
+    const int lane = threadIdx.x & 31, e1 = d.adjStart[g + 1];
+    int n = 0;
+    for (int e0 = d.adjStart[g]; e0 < e1; e0 += 32) {
+        const int mine = e0 + lane < e1 ? entryTerms(d, g, e0 + lane, [](int) { return 0u; }, [](int, const Term &) {}) : 0;
+        int upTo = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, upTo, o);
+            if (lane >= o)
+                upTo += y;
+        }
+        const int from = n + upTo - mine;
+        if (e0 + lane < e1)
+            entryTerms(d, g, e0 + lane, recOf, [&](int k, const Term &t) { put(from + k, t); });
+        n += __shfl_sync(0xffffffffu, upTo, 31);
+    }
+    return n;
 }
 
 // The first force whose body B is in slot `g` or later (forces lie in world order, as bodies do).
@@ -1108,8 +1514,100 @@ __device__ __forceinline__ int manifoldFlags(const Dev &d, int2 ab, int n) {
 
 struct SetupShared {
     int fits[kMaxTeam], active[kMaxTeam], entry0[kMaxTeam];
-    int tasks;
+    int tasks, colourCount[kMaxColours + 1], colourBase[kMaxColours + 1];
 };
+
+// Deals the world's coloured bodies, by colour and then slot, round the CTAs; a world's CTAs find the same.
+__device__ __forceinline__ void dealColours(const Dev &d, World &w, unsigned char *smem, SetupShared &sh, bool fits) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+    int *warpColours = arrayAt<int>(smem, 0) + warp * (kMaxColours + 1); // scratch
+    const auto colourOf = [&](int i) {
+        return i < w.cnt && inUpdate(d, w.base + i) && d.colour[w.base + i] < kMaxColours ? d.colour[w.base + i] : kMaxColours;
+    };
+    if (threadIdx.x <= kMaxColours)
+        sh.colourCount[threadIdx.x] = 0;
+    __syncthreads();
+    for (int i = threadIdx.x; i < w.cnt; i += blockDim.x)
+        if (colourOf(i) < kMaxColours)
+            atomicAdd(&sh.colourCount[colourOf(i)], 1);
+    __syncthreads();
+    int start = 0;
+    for (int c = 0; c <= kMaxColours; c++) { // the first of this CTA at or after the colour's start
+        w.colourAt[c] = (start - w.rank + w.size - 1) / w.size;
+        w.groupAt[c] = 0;
+        if (threadIdx.x == 0)
+            sh.colourBase[c] = start;
+        start += c < kMaxColours ? sh.colourCount[c] : 0;
+    }
+    for (int i0 = 0; i0 < w.cnt; i0 += blockDim.x) {
+        const int i = i0 + static_cast<int>(threadIdx.x), c = colourOf(i);
+        if (lane <= kMaxColours)
+            warpColours[lane] = 0;
+        __syncwarp();
+        const unsigned peers = __match_any_sync(0xffffffffu, c);
+        const int below = __popc(peers & ((1u << lane) - 1));
+        if (below == 0)
+            warpColours[c] = __popc(peers);
+        __syncthreads();
+        if (threadIdx.x < kMaxColours) {
+            int at = sh.colourBase[threadIdx.x];
+            for (int k = 0; k < warps; k++) {
+                int &n = arrayAt<int>(smem, 0)[k * (kMaxColours + 1) + threadIdx.x];
+                const int first = at;
+                at += n;
+                n = first;
+            }
+            sh.colourBase[threadIdx.x] = at;
+        }
+        __syncthreads();
+        if (fits && c < kMaxColours) {
+            const int at = warpColours[c] + below;
+            if (at % w.size == w.rank)
+                arrayAt<uint16_t>(smem, w.colourList)[at / w.size] = static_cast<uint16_t>(i);
+        }
+        __syncthreads();
+    }
+}
+
+// The terms of this CTA's coloured bodies and, a group at a time, their order by kind.
+__device__ __forceinline__ void listTerms(const Dev &d, const World &w, unsigned char *smem) {
+    const uint16_t *list = arrayAt<uint16_t>(smem, w.colourList);
+    const int *termFirst = arrayAt<int>(smem, w.termFirst);
+    Term *terms = arrayAt<Term>(smem, w.terms);
+    const int bodies = w.colourAt[kMaxColours];
+    for (int k = threadIdx.x >> 5; k < bodies; k += blockDim.x >> 5) {
+        const int first = termFirst[k];
+        bodyTerms(
+                d, w.base + list[k], [&](int b) { return placeOf(w, b - w.base).rec; },
+                [&](int n, const Term &t) {
+                    terms[first + n] = t;
+                    terms[first + n].row = first + n;
+                });
+    }
+    __syncthreads();
+    const int rows = passRows();
+    for (int c = 0; c < kMaxColours; c++) {
+        const int first = termFirst[w.colourAt[c]], last = termFirst[w.colourAt[c + 1]];
+        for (int e = first + static_cast<int>(threadIdx.x); e < last; e += blockDim.x) {
+            const int from = e - (e - first) % rows, to = min(from + rows, last), kind = terms[e].flags & kTermKind;
+            int at = from;
+            for (int k = from; k < to; k++) {
+                const int other = terms[k].flags & kTermKind;
+                at += other < kind || (other == kind && k < e) ? 1 : 0;
+            }
+            arrayAt<uint16_t>(smem, w.termOrder)[at] = static_cast<uint16_t>(e);
+        }
+        const int groups = w.groupAt[c + 1] - w.groupAt[c];
+        for (int k = threadIdx.x; k < groups * (kTermKinds + 1); k += blockDim.x) {
+            const int g = k / (kTermKinds + 1), kind = k - g * (kTermKinds + 1), from = first + g * rows, to = min(from + rows, last);
+            int before = 0;
+            for (int e = from; e < to; e++)
+                before += (terms[e].flags & kTermKind) < kind ? 1 : 0;
+            arrayAt<uint16_t>(smem, w.termKinds)[w.groupAt[c] * (kTermKinds + 1) + k] = static_cast<uint16_t>(before);
+        }
+    }
+}
+
 
 __device__ __forceinline__ int carve(int &at, size_t bytes) {
     const int p = at;
@@ -1120,7 +1618,7 @@ __device__ __forceinline__ int carve(int &at, size_t bytes) {
 // This CTA's part of the world, its state loaded; agrees with the cluster's other CTAs whether every
 // part fits in shared memory (false: the world is left to worldWideKernel) and whether any manifold
 // is active (`active`).
-template <bool ARM>
+template <bool ARM, bool COLOURS>
 __device__ __forceinline__ bool setupWorld(const Dev &d, const WorldRun &r, World &shared, unsigned char *smem, SetupShared &sh,
                                            bool &active) {
     const ManifoldBuf &L = d.live;
@@ -1147,6 +1645,10 @@ __device__ __forceinline__ bool setupWorld(const Dev &d, const WorldRun &r, Worl
     w.info = carve(at, sizeof(int) * w.per);
     w.entry = carve(at, sizeof(int) * (w.per + 1));
     w.rec = carve(at, kF4 * kRecF4 * w.per);
+    w.rec0 = static_cast<int>(sharedAddress(smem + w.rec));
+    w.con0 = static_cast<int>(sharedAddress(smem + w.con));
+    w.colourList = carve(at, COLOURS ? sizeof(uint16_t) * w.per : 0);
+    w.termFirst = carve(at, COLOURS ? sizeof(int) * (w.per + 1) : 0);
     w.stamps = carve(at, fits ? kF4 * kStampF4 * ne : 0);
     const int nm = fits ? w.nm : 0;
     w.mf = carve(at, sizeof(int2) * nm);
@@ -1200,6 +1702,38 @@ __device__ __forceinline__ bool setupWorld(const Dev &d, const WorldRun &r, Worl
         w.contacts = carve(at, static_cast<size_t>(ARM ? 7 : 5) * w.conStride);
         fits = at <= end;
     }
+    if (COLOURS) {
+        dealColours(d, w, smem, sh, fits);
+        w.colourBlocks = carve(at, sizeof(real) * kBlkReals * w.colourAt[kMaxColours]);
+        fits = fits && at <= end;
+        if (fits) {
+            int *termFirst = arrayAt<int>(smem, w.termFirst), *count = arrayAt<int>(smem, w.sums); // scratch
+            const int bodies = w.colourAt[kMaxColours];
+            for (int k = threadIdx.x >> 5; k < bodies; k += blockDim.x >> 5) {
+                const int n = bodyTerms(d, w.base + arrayAt<uint16_t>(smem, w.colourList)[k], [](int) { return 0u; }, [](int, const Term &) {});
+                if ((threadIdx.x & 31) == 0)
+                    count[k] = n;
+            }
+            __syncthreads();
+            for (int k = threadIdx.x; k <= bodies; k += blockDim.x) {
+                int before = 0;
+                for (int j = 0; j < k; j++)
+                    before += count[j];
+                termFirst[k] = before;
+            }
+            __syncthreads();
+            const int terms = termFirst[bodies];
+            for (int c = 0; c < kMaxColours; c++) {
+                const int n = termFirst[w.colourAt[c + 1]] - termFirst[w.colourAt[c]];
+                w.groupAt[c + 1] = w.groupAt[c] + max(1, (n + passRows() - 1) / passRows());
+            }
+            w.termKinds = carve(at, sizeof(uint16_t) * (kTermKinds + 1) * w.groupAt[kMaxColours]);
+            w.termOrder = carve(at, sizeof(uint16_t) * terms);
+            fits = terms < 65536 && at <= end;
+            w.terms = carve(at, fits ? sizeof(Term) * terms : 0);
+            fits = fits && at <= end;
+        }
+    }
     if (static_cast<int>(threadIdx.x) < w.size) {
         storeClusterInt(mapShared(sharedAddress(&sh.fits[w.rank]), threadIdx.x), fits ? 1 : 0);
         storeClusterInt(mapShared(sharedAddress(&sh.active[w.rank]), threadIdx.x), active ? 1 : 0);
@@ -1222,7 +1756,7 @@ __device__ __forceinline__ bool setupWorld(const Dev &d, const WorldRun &r, Worl
         const real4 x4 = d.x[g];
         const bool update = inUpdate(d, g);
         info[i] = (d.colour[g] & kBiColour) | (update ? kBiUpdate : 0) | (update && x4.w > 0.0f ? kBiMovable : 0) |
-                  (d.meta[g].w & 0xffff) << kBiLocks;
+                  (COLOURS && bodyHasForce(d, g, nForcesDev(d)) ? kBiForce : 0) | (d.meta[g].w & 0xffff) << kBiLocks;
         real4 *rec = arrayAt<real4>(smem, w.rec) + kRecF4 * i;
         rec[kRecX] = x4;
         rec[kRecQ] = d.q[g];
@@ -1278,6 +1812,8 @@ __device__ __forceinline__ bool setupWorld(const Dev &d, const WorldRun &r, Worl
             at(6) = L.armB[ci];
         }
     }
+    if (COLOURS)
+        listTerms(d, w, smem);
     if (threadIdx.x == 0)
         shared = w;
     clusterSync(w.size);
@@ -1322,6 +1858,7 @@ __global__ void __launch_bounds__(kMaxWorldThreads, 1)
     pdlTrigger();
     extern __shared__ __align__(32) unsigned char smem[];
     __shared__ int shared[4], deepest[2];
+    __shared__ real carry[32];
     __shared__ SetupShared sh;
     // The world's description is uniform and wide: it is kept in shared memory, and a phase reads what
     // it needs.
@@ -1373,7 +1910,7 @@ __global__ void __launch_bounds__(kMaxWorldThreads, 1)
             __syncthreads();
         }
         bool active;
-        const bool fits = setupWorld<ARM>(d, r, w, smem, sh, active);
+        const bool fits = setupWorld<ARM, COLOURS>(d, r, w, smem, sh, active);
         if (threadIdx.x == 0 && w.rank == 0)
             d.wStop[world] = fits ? 1 : 0; // 0: worldWideKernel's
         if (!fits)
@@ -1403,13 +1940,12 @@ __global__ void __launch_bounds__(kMaxWorldThreads, 1)
                 if (newton) {
                     if (COLOURS) {
                         if (colours) {
-                            colourPhase(d, p, w, smem, colours, it > 0 ? 1 : 0);
+                            colourPhase<ARM>(d, p, w, smem, colours, it > 0 ? 1 : 0, carry);
                             if (!bodyWarp())
                                 contactPhase<ARM, COLOURS>(d, p, w, smem, kStampsMixed, 1.0f);
                             clusterSync(size);
                         }
-                        startBlocks<true>(d, p, w, smem);
-                        __syncthreads();
+                        overflowForces(d, p, w, smem);
                     }
                     solvePhase<COLOURS>(d, p, w, smem);
                     clusterSync(size);
@@ -1422,12 +1958,10 @@ __global__ void __launch_bounds__(kMaxWorldThreads, 1)
                     contactPhase<ARM, COLOURS>(d, p, w, smem,
                                                it < 0 ? kStampsOverflow : (it + 1 < r.newtonRounds ? kDualStamps : kDual),
                                                newton || it < 0 ? 1.0f : p.stiffnessDecay);
-                if (!COLOURS && it + 1 < r.newtonRounds)
-                    startBlocks<false>(d, p, w, smem); // the poses of this phase are the next solve's
-                if (COLOURS && it >= 0)
-                    for (int f = w.f0 + w.rank * static_cast<int>(blockDim.x) + static_cast<int>(threadIdx.x); f < w.f1;
-                         f += size * static_cast<int>(blockDim.x))
-                        forceDualAt(d, p, f);
+                if (COLOURS && it >= 0 && bodyWarp())
+                    forceDuals(d, p, w);
+                if (it + 1 < r.newtonRounds)
+                    startBlocks<COLOURS>(p, w, smem); // the poses of this phase are where the next solve starts
                 clusterSync(size);
             }
             const int idle = step + 1 == r.substeps ? 1 : 0;
@@ -1631,14 +2165,16 @@ size_t worldRows(int threads) { return sizeof(real) * static_cast<size_t>(thread
 //                 not fit in shared memory, 1681 (walls) 637 / 551, 3000 (pile) 775 / 754
 //   many worlds   64 of 8-64 bodies 300 / 537, 256 of them 461 / 606, 512: 622 / 650, 1024: 945 / 751;
 //                 64 of 8-256 755 / 617
+//   with forces   600 bodies with ragdolls and springs 781 / 1680, a 1653-box pile with a chain 770 / 915
 // So worlds of up to 72 bodies a CTA, in up to three waves of CTAs, and a single world while it fits.
-bool worldsTake(int worlds, int bodies, double density) {
+bool worldsTake(int worlds, int bodies, double density, double forces) {
     const int team = worldTeam(worlds, bodies), per = divUp(bodies, team);
     if (worlds * team > 3 * kSms || (worlds > 1 && per > 72))
         return false;
     // Shared memory a CTA needs: its bodies, their stamp records (two a manifold), its manifolds and
     // their contacts (four a manifold and what packing leaves empty).
-    const double body = sizeof(real) * kBlkReals + kF4 * (kConF4 + kRecF4) + 8;
+    // With forces: a second block, and about eight terms a side of each.
+    const double body = sizeof(real) * kBlkReals * (forces > 0 ? 2 : 1) + kF4 * (kConF4 + kRecF4) + 8 + forces * 16 * (sizeof(Term) + 2);
     const double manifold = 2.0 * kF4 * kStampF4 + kF4 * 3 + 28 + 4.7 * (kF4 * 5 + 2);
     return worldRows(worldThreads(team, bodies)) + per * (body + density * manifold) < 0.99 * kSmemMost;
 }

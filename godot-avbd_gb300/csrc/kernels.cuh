@@ -100,9 +100,9 @@ struct WorldRun {
     unsigned rowBytes, smemBytes; // set by the launch
 };
 int worldTeamMax();
-// Whether a store of up to `worlds` worlds of up to `bodies` bodies, with about `density` manifolds a
-// body, is stepped this way.
-bool worldsTake(int worlds, int bodies, double density);
+// Whether a store of up to `worlds` worlds of up to `bodies` bodies, with about `density` manifolds and
+// `forces` forces a body, is stepped this way.
+bool worldsTake(int worlds, int bodies, double density, double forces);
 // `worlds`: at least the store's worlds; `bodies`: at least the largest one's.
 void launchWorlds(const Dev &d, const StepParams &p, const WorldRun &run, int worlds, int bodies, cudaStream_t s);
 

@@ -109,3 +109,73 @@ def test_wide_plate(pkg, gpu, oracle, boxes, last):
     d = capi.make_body_descs(*[sum((list(p[k]) for p in parts), []) for k in (0, 1)], 0.5,
                              sum((list(p[2]) for p in parts), []))
     assert same(run(gpu, capi, d, 25), run(oracle, capi, d, 25))
+
+
+def tangle(capi, n, seed, ragdolls=True):
+    """A heap with every kind of force among its bodies: a hub that carries most of them (more terms
+    than a warp has lanes), chains, world anchors, springs and, with `ragdolls`, soft joints and
+    free, limited and sprung rotations (of which the oracle may have other last bits)."""
+    d = heap(capi, n, seed)
+    at = lambda i: np.array(d[i].position[:])
+    lock, free = (1, 0, 0, 0, 0, 0), (0, 0, 0, 0, 0, 0)
+    hinge = free if ragdolls else lock
+    rng = np.random.default_rng(seed)
+    forces = []
+    for i in range(2, n + 1):
+        a = 1 if i % 2 else i - 1  # the hub, or a chain
+        r = tuple(0.5 * (at(i) - at(a)))
+        ends = (a, i, r, tuple(-x for x in r))
+        kind = i % 7
+        if kind == 0:
+            forces.append(("spring", *ends, 40.0, -1.0 if i % 3 else 0.7))
+        elif kind == 1:
+            forces.append(("generic", *ends, (lock, lock, lock, hinge, lock, lock)))
+        elif kind == 2 and ragdolls:
+            forces.append(("generic", *ends, (lock, lock, (0, 0, 0, 60.0, 0.1, 1.5), (2, -0.3, 0.3, 0, 0, 0),
+                                              (0, 0, 0, 40.0, 0.2, 2.0), lock)))
+        elif kind == 3:
+            forces.append(("generic", -1, i, tuple(at(i)), (0.0, 0.0, 0.0), (lock, (2, -0.5, 0.1, 0, 0, 0), free, hinge, hinge, hinge)))
+        elif kind == 4:
+            forces.append((*ends, *((800.0, 30.0) if ragdolls else (float("inf"), 0.0)), float("inf")))
+        elif kind == 5 and rng.random() < 0.5:
+            forces.append(("ignore", a, i))
+        else:
+            forces.append((*ends, float("inf"), 0.0, float("inf")))
+    return d, forces
+
+
+def run_forces(api, capi, world, params, steps=20, interleaved=None):
+    d, forces = world
+    p = api.default_params()
+    for k, v in params.items():
+        setattr(p, k, v)
+    w = capi.World(api, p, max_bodies=16384, max_forces=max(1, len(forces)))
+    w.add_bodies(d)
+    for f in forces:
+        w.add_force(f)
+    out = []
+    for _ in range(steps):
+        w.step_interleaved(*interleaved) if interleaved else w.step()
+        out.append(w.state())
+    return out
+
+
+# Forces on one CTA and on two, against the oracle.
+@pytest.mark.parametrize("n", [2, 9, 47])
+def test_forces(pkg, gpu, oracle, n):
+    capi = pkg.capi
+    world = tangle(capi, n, n, ragdolls=False)
+    assert same(run_forces(gpu, capi, world, {}), run_forces(oracle, capi, world, {}))
+
+
+# Every force, up to the largest cluster, arms kept from the dual, substeps, no projection: the same bits
+# as the separate launches.
+@pytest.mark.parametrize("n,params,interleaved", [
+    (12, {}, None), (47, {}, None), (200, {}, None), (400, {}, None), (130, {"jacobian_rebuild_distance": 0.05}, None),
+    (60, {"iterations": 3, "position_projection": 0}, (2, 3))])
+def test_forces_as_separate_launches(pkg, gpu, monkeypatch, n, params, interleaved):
+    capi = pkg.capi
+    world = tangle(capi, n, n)
+    here = run_forces(gpu, capi, world, params, interleaved=interleaved)
+    monkeypatch.setenv("AVBDG_NO_WORLD", "1")
+    assert same(here, run_forces(gpu, capi, world, params, interleaved=interleaved))
