@@ -161,85 +161,216 @@ __global__ void scanDownKernel(const int *in, int *out, int capacity, const int 
 }
 
 // ---------------------------------------------------------------------------------------------
-// Radix sort: 8-bit digits, 256 threads x 8 rounds per tile, stable ranking by warp matching.
+// Radix sort: 8-bit digits, tiles of 256 threads x 8 keys, stable ranking by warp votes.
+//
+// A pass counts each tile's digits, scans the counts along the tiles (a block a digit) and scatters.
+// In the scatter a warp ranks its 256 consecutive keys without meeting the others; the tile is then
+// put in digit order in shared memory, so neighbouring lanes write neighbouring keys, and every tile
+// finds the digits' bases from their 256 totals itself. A million keys a pass, kernels alone: 24.6 us
+// when each of eight rounds met three block barriers and scattered from registers, with the counts
+// scanned as one array of 131,072; 15.4 us this way (16 MB through L2). A single tile (stores of up
+// to 2048 bodies) needs neither count nor scan: one launch a pass.
 // ---------------------------------------------------------------------------------------------
 
 constexpr int kRadixThreads = 256;
+constexpr int kRadixWarps = kRadixThreads / 32;
 constexpr int kRadixRounds = 8;
 constexpr int kRadixTile = kRadixThreads * kRadixRounds;
 constexpr int kRadixBins = 256;
 
-__global__ void radixHistKernel(const uint64_t *keys, int capacity, const int *d_n, int shift, uint32_t mask,
-                                int numBlocks, int *hist) {
+// A tile's counts, at hist[digit * numBlocks + tile].
+__global__ void __launch_bounds__(kRadixThreads) radixHistKernel(const uint64_t *keys, int capacity, const int *d_n, int shift,
+                                                                 uint32_t mask, int numBlocks, int *hist) {
     pdlWait();
     pdlTrigger();
     __shared__ int h[kRadixBins];
     h[threadIdx.x] = 0;
     __syncthreads();
     const int n = loadCount(d_n, capacity);
-    const int base = blockIdx.x * kRadixTile;
-    for (int r = 0; r < kRadixRounds; r++) {
-        const int i = base + r * kRadixThreads + threadIdx.x;
-        if (i < n)
-            atomicAdd(&h[(keys[i] >> shift) & mask], 1);
-    }
+    const int base = blockIdx.x * kRadixTile + threadIdx.x;
+    uint64_t key[kRadixRounds];
+#pragma unroll
+    for (int r = 0; r < kRadixRounds; r++)
+        key[r] = base + r * kRadixThreads < n ? keys[base + r * kRadixThreads] : 0;
+#pragma unroll
+    for (int r = 0; r < kRadixRounds; r++)
+        if (base + r * kRadixThreads < n)
+            atomicAdd(&h[(key[r] >> shift) & mask], 1);
     __syncthreads();
     hist[threadIdx.x * numBlocks + blockIdx.x] = h[threadIdx.x];
 }
 
-__global__ void radixScatterKernel(const uint64_t *keysIn, const uint32_t *valsIn, uint64_t *keysOut,
-                                   uint32_t *valsOut, int capacity, const int *d_n, int shift, uint32_t mask,
-                                   int numBlocks, const int *offsets) {
+// Block d: the exclusive prefix of digit d's counts along the tiles, in place, and their total.
+__global__ void __launch_bounds__(kRadixThreads) radixScanKernel(int *hist, int numBlocks, int *totals) {
     pdlWait();
     pdlTrigger();
-    __shared__ int running[kRadixBins];
-    __shared__ int warpCount[kRadixThreads / 32][kRadixBins];
-    __shared__ int roundTotal[kRadixBins];
-    const int n = loadCount(d_n, capacity);
-    const int lane = threadIdx.x & 31;
-    const int warp = threadIdx.x >> 5;
-    running[threadIdx.x] = offsets[threadIdx.x * numBlocks + blockIdx.x];
-    const int base = blockIdx.x * kRadixTile;
-    const uint32_t ltMask = (1u << lane) - 1u;
-    for (int r = 0; r < kRadixRounds; r++) {
-        for (int w = 0; w < kRadixThreads / 32; w++)
-            warpCount[w][threadIdx.x] = 0;
-        __syncthreads();
-        const int i = base + r * kRadixThreads + threadIdx.x;
-        const bool valid = i < n;
-        uint64_t key = 0;
-        uint32_t val = 0;
-        uint32_t d = 0xffffffffu;
-        if (valid) {
-            key = keysIn[i];
-            val = valsIn ? valsIn[i] : 0u;
-            d = static_cast<uint32_t>((key >> shift) & mask);
+    __shared__ int warpSums[kRadixWarps];
+    constexpr int kItems = 4;
+    int *row = hist + static_cast<size_t>(blockIdx.x) * numBlocks;
+    int run = 0;
+    for (int first = 0; first < numBlocks; first += kRadixThreads * kItems) {
+        const int base = first + threadIdx.x * kItems;
+        int v[kItems], s = 0;
+#pragma unroll
+        for (int k = 0; k < kItems; k++) {
+            v[k] = base + k < numBlocks ? row[base + k] : 0;
+            s += v[k];
         }
-        const uint32_t peers = __match_any_sync(0xffffffffu, d);
-        const int rank = __popc(peers & ltMask);
-        if (valid && rank == 0)
-            warpCount[warp][d] = __popc(peers);
-        __syncthreads();
-        {
-            int acc = 0;
-            for (int w = 0; w < kRadixThreads / 32; w++) {
-                const int c = warpCount[w][threadIdx.x];
-                warpCount[w][threadIdx.x] = acc;
-                acc += c;
-            }
-            roundTotal[threadIdx.x] = acc;
+        int total;
+        int prefix = run + blockExclusiveScan<kRadixThreads>(s, warpSums, total);
+#pragma unroll
+        for (int k = 0; k < kItems; k++) {
+            if (base + k < numBlocks)
+                row[base + k] = prefix;
+            prefix += v[k];
         }
-        __syncthreads();
-        if (valid) {
-            const int pos = running[d] + warpCount[warp][d] + rank;
-            keysOut[pos] = key;
-            if (valsOut)
-                valsOut[pos] = val;
-        }
-        __syncthreads();
-        running[threadIdx.x] += roundTotal[threadIdx.x];
-        __syncthreads();
+        run += total;
     }
+    if (threadIdx.x == 0)
+        totals[blockIdx.x] = run;
+}
+
+__global__ void __launch_bounds__(kRadixThreads)
+        radixScatterKernel(const uint64_t *keysIn, const uint32_t *valsIn, uint64_t *keysOut, uint32_t *valsOut, int capacity,
+                           const int *d_n, int shift, uint32_t mask, int numBlocks, const int *hist, const int *totals) {
+    pdlWait();
+    pdlTrigger();
+    __shared__ int warpCount[kRadixWarps][kRadixBins];
+    __shared__ int place[kRadixBins]; // a digit's place in the output, less its place in the tile
+    __shared__ int warpSums[kRadixWarps];
+    __shared__ uint64_t tileKeys[kRadixTile];
+    __shared__ uint32_t tileVals[kRadixTile];
+    const int n = loadCount(d_n, capacity);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int first = static_cast<int>(blockIdx.x) * kRadixTile, base = first + warp * (32 * kRadixRounds) + lane;
+    uint64_t key[kRadixRounds];
+    uint32_t val[kRadixRounds];
+#pragma unroll
+    for (int r = 0; r < kRadixRounds; r++) {
+        const int i = base + 32 * r;
+        key[r] = i < n ? keysIn[i] : 0;
+        val[r] = i < n && valsIn ? valsIn[i] : 0u;
+    }
+    for (int b = lane; b < kRadixBins; b += 32)
+        warpCount[warp][b] = 0;
+    __syncwarp();
+    // Each key's rank among the warp's earlier keys of its digit.
+    int rank[kRadixRounds];
+#pragma unroll
+    for (int r = 0; r < kRadixRounds; r++) {
+        const bool valid = base + 32 * r < n;
+        const uint32_t d = static_cast<uint32_t>((key[r] >> shift) & mask);
+        uint32_t peers = __ballot_sync(0xffffffffu, valid);
+#pragma unroll
+        for (int b = 0; b < 8; b++) { // (eight votes take less than one match of scattered digits)
+            const uint32_t ones = __ballot_sync(0xffffffffu, (d >> b) & 1u);
+            peers &= (d >> b) & 1u ? ones : ~ones;
+        }
+        const int below = __popc(peers & ((1u << lane) - 1u));
+        rank[r] = valid ? warpCount[warp][d] + below : 0;
+        __syncwarp();
+        if (valid && below == 0)
+            warpCount[warp][d] += __popc(peers);
+        __syncwarp();
+    }
+    __syncthreads();
+    // Thread b: digit b's warps in order, its place in the tile and in the output.
+    {
+        int mine = 0;
+#pragma unroll
+        for (int w = 0; w < kRadixWarps; w++) {
+            const int c = warpCount[w][threadIdx.x];
+            warpCount[w][threadIdx.x] = mine;
+            mine += c;
+        }
+        int total;
+        const int inTile = blockExclusiveScan<kRadixThreads>(mine, warpSums, total);
+        int out = inTile;
+        if (numBlocks > 1)
+            out = blockExclusiveScan<kRadixThreads>(totals[threadIdx.x], warpSums, total) +
+                  hist[threadIdx.x * numBlocks + blockIdx.x];
+#pragma unroll
+        for (int w = 0; w < kRadixWarps; w++)
+            warpCount[w][threadIdx.x] += inTile;
+        place[threadIdx.x] = out - inTile;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kRadixRounds; r++)
+        if (base + 32 * r < n) {
+            const int at = warpCount[warp][(key[r] >> shift) & mask] + rank[r];
+            tileKeys[at] = key[r];
+            tileVals[at] = val[r];
+        }
+    __syncthreads();
+    const int count = min(kRadixTile, n - first);
+#pragma unroll
+    for (int r = 0; r < kRadixRounds; r++) {
+        const int i = r * kRadixThreads + threadIdx.x;
+        if (i < count) {
+            const uint64_t k = tileKeys[i];
+            const int to = place[(k >> shift) & mask] + i;
+            keysOut[to] = k;
+            if (valsOut)
+                valsOut[to] = tileVals[i];
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------------------------
+// The distinct keys of a sorted array: a key counts where it differs from the one before. Both passes
+// read the keys (the second from L2) rather than keep a flag and a rank for each.
+// ---------------------------------------------------------------------------------------------
+
+__device__ __forceinline__ bool firstOfKey(const uint64_t *keys, int i, int n) { return i < n && (i == 0 || keys[i] != keys[i - 1]); }
+
+__global__ void __launch_bounds__(kRadixThreads) uniqueCountKernel(const uint64_t *keys, int n, int *blockSums) {
+    pdlWait();
+    pdlTrigger();
+    __shared__ int warpSums[kRadixWarps];
+    const int base = blockIdx.x * kRadixTile + threadIdx.x;
+    int mine = 0;
+#pragma unroll
+    for (int r = 0; r < kRadixRounds; r++)
+        mine += firstOfKey(keys, base + r * kRadixThreads, n) ? 1 : 0;
+    int total;
+    blockExclusiveScan<kRadixThreads>(mine, warpSums, total);
+    if (threadIdx.x == 0)
+        blockSums[blockIdx.x] = total;
+}
+
+__global__ void __launch_bounds__(kRadixThreads) uniqueScatterKernel(const uint64_t *keys, int n, const int *blockSums, uint64_t *out) {
+    pdlWait();
+    pdlTrigger();
+    __shared__ int counts[kRadixRounds * kRadixWarps];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, base = blockIdx.x * kRadixTile + threadIdx.x;
+    unsigned hits[kRadixRounds];
+#pragma unroll
+    for (int r = 0; r < kRadixRounds; r++) {
+        hits[r] = __ballot_sync(0xffffffffu, firstOfKey(keys, base + r * kRadixThreads, n));
+        if (lane == 0)
+            counts[r * kRadixWarps + warp] = __popc(hits[r]);
+    }
+    __syncthreads();
+    if (warp == 0) { // two counts a lane
+        static_assert(kRadixRounds * kRadixWarps == 64, "two counts a lane");
+        const int a = counts[2 * lane], b = counts[2 * lane + 1];
+        int upTo = a + b;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, upTo, o);
+            if (lane >= o)
+                upTo += y;
+        }
+        const int before = blockSums[blockIdx.x] + upTo - a - b;
+        counts[2 * lane] = before;
+        counts[2 * lane + 1] = before + a;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kRadixRounds; r++)
+        if ((hits[r] >> lane) & 1u)
+            out[counts[r * kRadixWarps + warp] + __popc(hits[r] & ((1u << lane) - 1u))] = keys[base + r * kRadixThreads];
 }
 
 template <typename T>
@@ -369,9 +500,10 @@ size_t scanScratchBytes(int capacity) {
 
 size_t radixScratchBytes(int capacity) {
     const int blocks = divUp(capacity > 0 ? capacity : 1, kRadixTile);
-    const int histN = blocks * kRadixBins;
-    return static_cast<size_t>(histN) * sizeof(int) + scanScratchBytes(histN) + 256;
+    return (static_cast<size_t>(blocks) + 1) * kRadixBins * sizeof(int);
 }
+
+size_t uniqueScratchBytes(int count) { return static_cast<size_t>(divUp(count > 0 ? count : 1, kRadixTile)) * sizeof(int); }
 
 void scanExclusive(const int *in, int *out, int capacity, const int *d_n, int *d_total, void *scratch,
                    cudaStream_t stream) {
@@ -389,19 +521,22 @@ void scanExclusive(const int *in, int *out, int capacity, const int *d_n, int *d
 void radixSortPairs(uint64_t *keys, uint32_t *values, uint64_t *keysAlt, uint32_t *valuesAlt, int capacity,
                     const int *d_n, int beginBit, int endBit, void *scratch, cudaStream_t stream) {
     const int blocks = divUp(capacity > 0 ? capacity : 1, kRadixTile);
-    const int histN = blocks * kRadixBins;
-    int *hist = static_cast<int *>(scratch);
-    void *scanScratch = reinterpret_cast<char *>(scratch) + static_cast<size_t>(histN) * sizeof(int) + 128;
+    int *totals = static_cast<int *>(scratch), *hist = totals + kRadixBins;
     uint64_t *kin = keys, *kout = keysAlt;
     uint32_t *vin = values, *vout = valuesAlt;
     int passes = 0;
     for (int bit = beginBit; bit < endBit; bit += 8) {
         const int bits = endBit - bit < 8 ? endBit - bit : 8;
         const uint32_t mask = (1u << bits) - 1u;
-        ++launchCount(); launchK(radixHistKernel, blocks, kRadixThreads, 0, stream, kin, capacity, d_n, bit, mask, blocks, hist);
-        scanExclusive(hist, hist, histN, nullptr, nullptr, scanScratch, stream);
-        ++launchCount(); launchK(radixScatterKernel, blocks, kRadixThreads, 0, stream, kin, vin, kout, vout, capacity, d_n, bit, mask,
-                                                                 blocks, hist);
+        if (blocks > 1) {
+            ++launchCount();
+            launchK(radixHistKernel, blocks, kRadixThreads, 0, stream, kin, capacity, d_n, bit, mask, blocks, hist);
+            ++launchCount();
+            launchK(radixScanKernel, kRadixBins, kRadixThreads, 0, stream, hist, blocks, totals);
+        }
+        ++launchCount();
+        launchK(radixScatterKernel, blocks, kRadixThreads, 0, stream, kin, vin, kout, vout, capacity, d_n, bit, mask, blocks, hist,
+                totals);
         uint64_t *tk = kin;
         kin = kout;
         kout = tk;
@@ -418,6 +553,14 @@ void radixSortPairs(uint64_t *keys, uint32_t *values, uint64_t *keysAlt, uint32_
             launchK(copyKernel<uint32_t>, grid, 256, 0, stream, vin, values, capacity, d_n);
         }
     }
+}
+
+void uniqueSorted(const uint64_t *keys, int n, uint64_t *out, int *d_count, void *scratch, cudaStream_t stream) {
+    const int blocks = divUp(n, kRadixTile);
+    int *blockSums = static_cast<int *>(scratch);
+    ++launchCount(); launchK(uniqueCountKernel, blocks, kRadixThreads, 0, stream, keys, n, blockSums);
+    ++launchCount(); launchK(scanTopKernel, 1, kTopThreads, 0, stream, blockSums, blocks, d_count);
+    ++launchCount(); launchK(uniqueScatterKernel, blocks, kRadixThreads, 0, stream, keys, n, blockSums, out);
 }
 
 template <typename T>

@@ -56,6 +56,10 @@ inline void launchK(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem
 // Scratch sizes the primitives need for `capacity` elements.
 size_t scanScratchBytes(int capacity);
 size_t radixScratchBytes(int capacity);
+size_t uniqueScratchBytes(int count);
+
+// out = the distinct keys of the sorted keys[0, n), n > 0; *d_count = how many.
+void uniqueSorted(const uint64_t *keys, int n, uint64_t *out, int *d_count, void *scratch, cudaStream_t stream);
 
 // out[i] = sum(in[0..i)) for i < *d_n; *d_total = sum(in[0..*d_n)) (d_total may be null).
 // `in` and `out` may alias.

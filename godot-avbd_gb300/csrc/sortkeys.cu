@@ -20,22 +20,6 @@ int sortFail(int code, const std::string &msg) {
     return code;
 }
 
-__global__ void uniqueFlagKernel(const uint64_t *keys, int n, int *flags) {
-    pdlWait();
-    pdlTrigger();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n)
-        flags[i] = (i == 0 || keys[i] != keys[i - 1]) ? 1 : 0;
-}
-
-__global__ void uniqueScatterKernel(const uint64_t *keys, int n, const int *flags, const int *rank, uint64_t *out) {
-    pdlWait();
-    pdlTrigger();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n && flags[i])
-        out[rank[i]] = keys[i];
-}
-
 __global__ void copyBackKernel(const uint64_t *src, uint64_t *dst, const int *count) {
     pdlWait();
     pdlTrigger();
@@ -44,23 +28,35 @@ __global__ void copyBackKernel(const uint64_t *src, uint64_t *dst, const int *co
         dst[i] = src[i];
 }
 
-// Scratch of one call: alternate key buffer, radix histograms, flags, ranks, scan blocks, count.
+// Scratch of one call: alternate key buffer, radix counts, block sums of the unique pass, count.
 struct SortScratch {
     uint64_t *keysAlt;
     void *radix;
-    int *flags;
-    int *ranks;
-    void *scan;
+    void *unique;
     int *count;
+};
+
+// The places of a call's scratch for n keys in one block of `bytes`.
+struct SortLayout {
+    size_t radix, unique, count, bytes;
+    explicit SortLayout(int n) {
+        const auto up = [](size_t v) { return (v + 255) & ~size_t(255); };
+        radix = up(static_cast<size_t>(n) * sizeof(uint64_t));
+        unique = up(radix + radixScratchBytes(n));
+        count = up(unique + uniqueScratchBytes(n));
+        bytes = count + 256;
+    }
+    SortScratch at(void *base) const {
+        char *b = static_cast<char *>(base);
+        return SortScratch{reinterpret_cast<uint64_t *>(b), b + radix, b + unique, reinterpret_cast<int *>(b + count)};
+    }
 };
 
 // The sort + unique sequence, enqueued on `stream` with caller-provided scratch.
 void enqueueSortUnique(uint64_t *keys, int n, int bits, const SortScratch &s, cudaStream_t stream) {
     radixSortPairs(keys, nullptr, s.keysAlt, nullptr, n, nullptr, 0, bits, s.radix, stream);
+    uniqueSorted(keys, n, s.keysAlt, s.count, s.unique, stream);
     const int grid = divUp(n, 256);
-    launchK(uniqueFlagKernel, grid, 256, 0, stream, keys, n, s.flags);
-    scanExclusive(s.flags, s.ranks, n, nullptr, s.count, s.scan, stream);
-    launchK(uniqueScatterKernel, grid, 256, 0, stream, keys, n, s.flags, s.ranks, s.keysAlt);
     launchK(copyBackKernel, grid < 1184 ? grid : 1184, 256, 0, stream, s.keysAlt, keys, s.count);
 }
 
@@ -131,23 +127,15 @@ int avbdg_sort_unique_keys_static(uint64_t *d_keys, int count, int key_bits, int
         *unique_count = 0;
         return AVBDG_OK;
     }
-    const size_t n = static_cast<size_t>(count);
-    const size_t offAlt = 0;
-    const size_t offRadix = (offAlt + n * sizeof(uint64_t) + 255) & ~size_t(255);
-    const size_t offFlags = (offRadix + radixScratchBytes(count) + 255) & ~size_t(255);
-    const size_t offRanks = (offFlags + n * sizeof(int) + 255) & ~size_t(255);
-    const size_t offScan = (offRanks + n * sizeof(int) + 255) & ~size_t(255);
-    const size_t offCount = (offScan + scanScratchBytes(count) + 255) & ~size_t(255);
-    if (offCount + 256 > kStaticScratchBytes)
+    const SortLayout layout(count);
+    if (layout.bytes > kStaticScratchBytes)
         return sortFail(AVBDG_ERR_CAPACITY, "static sort scratch too small for this count");
     void *addr = nullptr;
     rc = staticScratchAddress(&addr);
     if (rc)
         return rc;
-    char *base = static_cast<char *>(addr);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    SortScratch s{reinterpret_cast<uint64_t *>(base + offAlt), base + offRadix, reinterpret_cast<int *>(base + offFlags),
-                  reinterpret_cast<int *>(base + offRanks), base + offScan, reinterpret_cast<int *>(base + offCount)};
+    const SortScratch s = layout.at(addr);
     // The array keeps whatever the previous call left. Every word this call reads is written by
     // it first (the scan's top kernel writes the count before copyBackKernel reads it); the
     // count is cleared as well, defensively.
@@ -176,19 +164,11 @@ int avbdg_sort_unique_keys(uint64_t *d_keys, int count, int key_bits, int *uniqu
         return AVBDG_OK;
     }
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const size_t n = static_cast<size_t>(count);
-    const size_t offAlt = 0;
-    const size_t offRadix = (offAlt + n * sizeof(uint64_t) + 255) & ~size_t(255);
-    const size_t offFlags = (offRadix + radixScratchBytes(count) + 255) & ~size_t(255);
-    const size_t offRanks = (offFlags + n * sizeof(int) + 255) & ~size_t(255);
-    const size_t offScan = (offRanks + n * sizeof(int) + 255) & ~size_t(255);
-    const size_t offCount = (offScan + scanScratchBytes(count) + 255) & ~size_t(255);
-    const size_t total = offCount + 256;
-    char *base = nullptr;
-    if (cudaMalloc(&base, total) != cudaSuccess)
+    const SortLayout layout(count);
+    void *base = nullptr;
+    if (cudaMalloc(&base, layout.bytes) != cudaSuccess)
         return sortFail(AVBDG_ERR_CAPACITY, "cudaMalloc of the sort scratch failed");
-    SortScratch s{reinterpret_cast<uint64_t *>(base + offAlt), base + offRadix, reinterpret_cast<int *>(base + offFlags),
-                  reinterpret_cast<int *>(base + offRanks), base + offScan, reinterpret_cast<int *>(base + offCount)};
+    const SortScratch s = layout.at(base);
     enqueueSortUnique(d_keys, count, key_bits, s, st);
     const cudaError_t launch = cudaPeekAtLastError();
     int host = 0;

@@ -52,3 +52,12 @@ def test_sort_unique_edge_cases(pkg):
     assert np.array_equal(_run(fn, pairs, 43), pairs)
     assert fn(None, 10, 64, ctypes.byref(out), None) == pkg.capi.ERR_INVALID
     assert fn(None, 0, 65, ctypes.byref(out), None) == pkg.capi.ERR_INVALID
+
+
+# Around a tile of 2048 keys and a thousand tiles, one digit and eight, all keys alike and all distinct.
+@pytest.mark.parametrize("n", [31, 2047, 2048, 2049, 4096, 70_001, 2_100_000])
+@pytest.mark.parametrize("bits,distinct", [(5, 32), (8, 3), (9, 512), (43, 1), (43, 1 << 30), (64, 1 << 40)])
+def test_sort_unique_tile_edges(pkg, n, bits, distinct):
+    rng = np.random.default_rng(n)
+    keys = rng.integers(0, distinct, size=n, dtype=np.uint64) << np.uint64(max(0, bits - distinct.bit_length() - 1))
+    assert np.array_equal(_run(_fn(pkg), keys, bits), np.unique(keys))
