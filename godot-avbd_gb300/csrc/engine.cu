@@ -262,6 +262,7 @@ Engine::~Engine() {
         cudaStreamSynchronize(stream);
     dropGraphs();
     releaseAll();
+    releaseSortScratch();
     if (ioHost)
         cudaFreeHost(ioHost);
     if (ctrRing)
@@ -294,8 +295,12 @@ template <typename T>
 T *Engine::dalloc(size_t n) {
     void *p = nullptr;
     const size_t bytes = std::max<size_t>(n, 1) * sizeof(T);
-    if (cudaMalloc(&p, bytes) != cudaSuccess)
-        return nullptr;
+    if (cudaMalloc(&p, bytes) != cudaSuccess) {
+        releaseSortScratch();
+        if (cudaMalloc(&p, bytes) != cudaSuccess)
+            return nullptr;
+        cudaGetLastError();
+    }
     cudaMemsetAsync(p, 0, bytes, stream);
     allocs.push_back(p);
     return static_cast<T *>(p);
@@ -1493,24 +1498,76 @@ int Engine::getSleeping(int w, int first, int count, uint8_t *out) {
 
 namespace {
 
-// Device scratch of one query call, released on every path.
-struct QueryScratch {
-    std::vector<void *> ptrs;
-    ~QueryScratch() {
-        for (void *p : ptrs)
-            cudaFree(p);
+// A query's place in device and host memory: the engine's kept blocks, or its own where another thread
+// is using them or it needs more than is kept.
+class QueryLease {
+public:
+    QueryLease(QueryScratch &scratch, size_t devBytes, size_t hostBytes) : kept(scratch), lock(scratch.mutex, std::try_to_lock) {
+        if (lock.owns_lock() && devBytes <= QueryScratch::kMost && hostBytes <= QueryScratch::kMost && kept.reserve(devBytes, hostBytes)) {
+            dev = static_cast<char *>(kept.dev);
+            host = static_cast<char *>(kept.host);
+            return;
+        }
+        cudaGetLastError(); // (of a block that could not grow)
+        if (cudaMalloc(&own, devBytes) != cudaSuccess) {
+            own = nullptr;
+            return;
+        }
+        pageable.resize(hostBytes);
+        dev = static_cast<char *>(own);
+        host = pageable.data();
     }
-    template <typename T>
-    T *get(size_t n) {
-        void *p = nullptr;
-        if (cudaMalloc(&p, std::max<size_t>(n, 1) * sizeof(T)) != cudaSuccess)
-            return nullptr;
-        ptrs.push_back(p);
-        return static_cast<T *>(p);
+    ~QueryLease() {
+        if (own)
+            cudaFree(own);
     }
+    char *dev = nullptr, *host = nullptr;
+
+private:
+    QueryScratch &kept;
+    std::unique_lock<std::mutex> lock;
+    void *own = nullptr;
+    std::vector<char> pageable;
 };
 
 } // namespace
+
+QueryScratch::~QueryScratch() {
+    if (dev)
+        cudaFree(dev);
+    if (host)
+        cudaFreeHost(host);
+}
+
+bool QueryScratch::reserve(size_t devWant, size_t hostWant) {
+    const auto grown = [](size_t want) {
+        size_t n = 65536;
+        while (n < want)
+            n *= 2;
+        return n;
+    };
+    if (devWant > devBytes) {
+        if (dev)
+            cudaFree(dev);
+        devBytes = 0;
+        if (cudaMalloc(&dev, grown(devWant)) != cudaSuccess) {
+            dev = nullptr;
+            return false;
+        }
+        devBytes = grown(devWant);
+    }
+    if (hostWant > hostBytes) {
+        if (host)
+            cudaFreeHost(host);
+        hostBytes = 0;
+        if (cudaMallocHost(&host, grown(hostWant)) != cudaSuccess) {
+            host = nullptr;
+            return false;
+        }
+        hostBytes = grown(hostWant);
+    }
+    return true;
+}
 
 int Engine::pick(int w, int count, const float *origins, const float *dirs, uint32_t mask, int *outBody,
                  float *outLocal) {
@@ -1518,29 +1575,27 @@ int Engine::pick(int w, int count, const float *origins, const float *dirs, uint
         return fail(AVBDG_ERR_INVALID, "bad pick arguments");
     if (count == 0)
         return AVBDG_OK;
-    std::vector<float> rays(6 * static_cast<size_t>(count));
-    for (int i = 0; i < count; i++)
-        for (int k = 0; k < 3; k++) {
-            rays[6 * i + k] = origins[3 * i + k];
-            rays[6 * i + 3 + k] = dirs[3 * i + k];
-        }
-    QueryScratch q;
-    float *dRays = q.get<float>(rays.size());
-    auto *dBest = q.get<unsigned long long>(count);
-    int *dBody = q.get<int>(count);
-    float *dLocal = q.get<float>(3 * static_cast<size_t>(count));
-    if (!dRays || !dBest || !dBody || !dLocal)
+    // Best hits, then the origins and directions, then the answers: bodies and local points.
+    const size_t n = static_cast<size_t>(count), rayBytes = sizeof(float) * 6 * n, outBytes = (sizeof(int) + 3 * sizeof(float)) * n;
+    QueryLease q(queryScratch, sizeof(unsigned long long) * n + rayBytes + outBytes, std::max(rayBytes, outBytes));
+    if (!q.dev)
         return fail(AVBDG_ERR_CAPACITY, "query scratch allocation failed");
+    auto *dBest = reinterpret_cast<unsigned long long *>(q.dev);
+    float *dRays = reinterpret_cast<float *>(dBest + n);
+    int *dBody = reinterpret_cast<int *>(dRays + 6 * n);
+    float *dLocal = reinterpret_cast<float *>(dBody + n);
+    std::memcpy(q.host, origins, rayBytes / 2);
+    std::memcpy(q.host + rayBytes / 2, dirs, rayBytes / 2);
     sync();
-    cudaMemcpyAsync(dRays, rays.data(), sizeof(float) * rays.size(), cudaMemcpyHostToDevice, stream);
+    cudaMemcpyAsync(dRays, q.host, rayBytes, cudaMemcpyHostToDevice, stream);
     launchPick(d, wBase[w], wCount[w], dRays, count, mask, dBest, dBody, dLocal, stream);
-    std::vector<float> local(3 * static_cast<size_t>(count));
-    cudaMemcpyAsync(outBody, dBody, sizeof(int) * static_cast<size_t>(count), cudaMemcpyDeviceToHost, stream);
-    cudaMemcpyAsync(local.data(), dLocal, sizeof(float) * local.size(), cudaMemcpyDeviceToHost, stream);
+    // (the stream has read the rays when it writes the answers over them)
+    cudaMemcpyAsync(q.host, dBody, outBytes, cudaMemcpyDeviceToHost, stream);
     if (cudaStreamSynchronize(stream) != cudaSuccess)
         return cudaCheck("pick");
+    std::memcpy(outBody, q.host, sizeof(int) * n);
     if (outLocal)
-        std::memcpy(outLocal, local.data(), sizeof(float) * local.size());
+        std::memcpy(outLocal, q.host + sizeof(int) * n, 3 * sizeof(float) * n);
     return cudaCheck("pick");
 }
 
@@ -1549,20 +1604,24 @@ int Engine::collectAabb(int w, const float lo[3], const float hi[3], uint32_t ma
     if (w < 0 || w >= worlds() || !lo || !hi || capacity < 0 || (capacity > 0 && !out))
         return fail(AVBDG_ERR_INVALID, "bad collect arguments");
     const int n = wCount[w];
-    QueryScratch q;
-    int *flags = q.get<int>(n), *rank = q.get<int>(n), *total = q.get<int>(1), *ids = q.get<int>(n);
-    if (!flags || !rank || !total || !ids)
+    const size_t room = static_cast<size_t>(std::max(n, 1));
+    const int most = std::min(n, capacity);
+    QueryLease q(queryScratch, sizeof(int) * (3 * room + 1), sizeof(int) * (room + 1));
+    if (!q.dev)
         return fail(AVBDG_ERR_CAPACITY, "query scratch allocation failed");
+    int *total = reinterpret_cast<int *>(q.dev), *ids = total + 1, *flags = ids + room, *rank = flags + room;
     sync();
     launchCollectAabb(d, wBase[w], n, f3{lo[0], lo[1], lo[2]}, f3{hi[0], hi[1], hi[2]}, mask, flags, rank, total,
                       d.scanScratch, n, ids, stream);
-    int found = 0;
-    cudaMemcpyAsync(&found, total, sizeof(int), cudaMemcpyDeviceToHost, stream);
+    // The count and as many ids as could be wanted, in one copy.
+    cudaMemcpyAsync(q.host, total, sizeof(int) * (1 + static_cast<size_t>(most)), cudaMemcpyDeviceToHost, stream);
     if (cudaStreamSynchronize(stream) != cudaSuccess)
         return cudaCheck("collectAabb");
+    int found = 0;
+    std::memcpy(&found, q.host, sizeof(int));
     const int k = std::min(found, capacity);
     if (k > 0)
-        cudaMemcpy(out, ids, sizeof(int) * static_cast<size_t>(k), cudaMemcpyDeviceToHost);
+        std::memcpy(out, q.host + sizeof(int), sizeof(int) * static_cast<size_t>(k));
     if (outCount)
         *outCount = found;
     return cudaCheck("collectAabb");

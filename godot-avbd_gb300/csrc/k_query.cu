@@ -73,6 +73,10 @@ __device__ real rayTest(const Dev &d, int g, f3 origin, f3 dir, f3 &local) {
     return tHit;
 }
 
+// The rays' origins, then their directions.
+__device__ __forceinline__ f3 rayOrigin(const float *rays, int r) { return f3{rays[3 * r], rays[3 * r + 1], rays[3 * r + 2]}; }
+__device__ __forceinline__ f3 rayDirection(const float *rays, int nRays, int r) { return rayOrigin(rays + 3 * static_cast<size_t>(nRays), r); }
+
 __global__ void pickResetKernel(unsigned long long *best, int rays) {
     pdlWait();
     pdlTrigger();
@@ -94,9 +98,8 @@ __global__ void pickKernel(Dev d, int base, int count, const float *rays, int nR
     const int g = base + static_cast<int>(t % count);
     if ((static_cast<unsigned>(d.meta[g].y) & mask) == 0)
         return;
-    const float *ray = rays + 6 * r;
     f3 local;
-    const real dist = rayTest(d, g, f3{ray[0], ray[1], ray[2]}, f3{ray[3], ray[4], ray[5]}, local);
+    const real dist = rayTest(d, g, rayOrigin(rays, r), rayDirection(rays, nRays, r), local);
     if (!(dist < bitsf(0x7f800000)))
         return;
     const unsigned bits = static_cast<unsigned>(fbits(dist + 0.0f));
@@ -118,9 +121,8 @@ __global__ void pickResultKernel(Dev d, int base, int count, const float *rays, 
         return;
     }
     const int g = base + (count - 1 - static_cast<int>(key & 0xffffffffu)); // list position -> slot
-    const float *ray = rays + 6 * r;
     f3 local{0, 0, 0};
-    rayTest(d, g, f3{ray[0], ray[1], ray[2]}, f3{ray[3], ray[4], ray[5]}, local);
+    rayTest(d, g, rayOrigin(rays, r), rayDirection(rays, nRays, r), local);
     outBody[r] = g - base;
     outLocal[3 * r] = local.x;
     outLocal[3 * r + 1] = local.y;

@@ -5,6 +5,9 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <utility>
+
+#include <cuda.h>
 
 #include "avbdg.h"
 #include "prims.cuh"
@@ -109,7 +112,97 @@ int staticScratchAddress(void **out) {
     return AVBDG_OK;
 }
 
+// ---- Kept scratch -----------------------------------------------------------------------------
+//
+// A cudaMalloc and a cudaFree of a million keys' scratch take about 155 us, more than the kernels do.
+// So a call leaves its block for the next one: at most one a device, of at most kKeptBytes. A
+// call takes the block out (a second thread finds none and allocates), and it has waited for its stream
+// before it puts it back, so no stream ever shares it. It belongs to the context it was allocated in, which
+// is known by its id: after a device reset it is forgotten. It is given back when a world, batch or server
+// is destroyed and when one of them cannot allocate.
+constexpr size_t kKeptBytes = size_t(64) << 20;
+
+struct KeptScratch {
+    void *base;
+    size_t bytes;
+    unsigned long long context;
+};
+static KeptScratch g_kept[kMaxDevices] = {};
+static std::mutex g_keptMutex;
+
+// The id of the current context, unique in the process; 0 where there is none.
+unsigned long long contextId() {
+    using Fn = CUresult (*)(CUcontext, unsigned long long *);
+    static const Fn fn = [] {
+        void *p = nullptr;
+        cudaDriverEntryPointQueryResult found = cudaDriverEntryPointSymbolNotFound;
+        const cudaError_t e = cudaGetDriverEntryPointByVersion("cuCtxGetId", &p, 12000, cudaEnableDefault, &found);
+        return reinterpret_cast<Fn>(e == cudaSuccess && found == cudaDriverEntryPointSuccess ? p : nullptr);
+    }();
+    unsigned long long id = 0;
+    return fn && fn(nullptr, &id) == CUDA_SUCCESS ? id : 0;
+}
+
+// Scratch for one call: the kept block of the current device if it is large enough, else a new one.
+class ScratchLease {
+public:
+    explicit ScratchLease(size_t bytes, cudaStream_t stream) {
+        // A stream in capture takes none: what is captured would use it later.
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        const bool plain = cudaStreamIsCapturing(stream, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone;
+        if (plain && cudaGetDevice(&device) == cudaSuccess && device >= 0 && device < kMaxDevices && (block.context = contextId())) {
+            KeptScratch kept{};
+            {
+                std::lock_guard<std::mutex> lock(g_keptMutex);
+                std::swap(kept, g_kept[device]);
+            }
+            if (kept.base && kept.context == block.context) {
+                if (kept.bytes >= bytes) {
+                    block = kept;
+                    return;
+                }
+                cudaFree(kept.base);
+            }
+        }
+        if (cudaMalloc(&block.base, bytes) != cudaSuccess)
+            block.base = nullptr;
+        block.bytes = bytes;
+    }
+    ~ScratchLease() {
+        if (block.base && block.context && block.bytes <= kKeptBytes && idle) {
+            std::lock_guard<std::mutex> lock(g_keptMutex);
+            if (!g_kept[device].base) {
+                g_kept[device] = block;
+                return;
+            }
+        }
+        if (block.base)
+            cudaFree(block.base);
+    }
+    ScratchLease(const ScratchLease &) = delete;
+    ScratchLease &operator=(const ScratchLease &) = delete;
+    void *base() const { return block.base; }
+    bool idle = false; // the stream has been waited for: the block may be kept
+
+private:
+    int device = 0;
+    KeptScratch block{};
+};
+
 } // namespace
+
+void releaseSortScratch() {
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= kMaxDevices)
+        return;
+    KeptScratch kept{};
+    {
+        std::lock_guard<std::mutex> lock(g_keptMutex);
+        std::swap(kept, g_kept[device]);
+    }
+    if (kept.base && kept.context == contextId())
+        cudaFree(kept.base);
+}
 
 } // namespace avbdg
 
@@ -165,16 +258,16 @@ int avbdg_sort_unique_keys(uint64_t *d_keys, int count, int key_bits, int *uniqu
     }
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const SortLayout layout(count);
-    void *base = nullptr;
-    if (cudaMalloc(&base, layout.bytes) != cudaSuccess)
+    ScratchLease scratch(layout.bytes, st);
+    if (!scratch.base())
         return sortFail(AVBDG_ERR_CAPACITY, "cudaMalloc of the sort scratch failed");
-    const SortScratch s = layout.at(base);
+    const SortScratch s = layout.at(scratch.base());
     enqueueSortUnique(d_keys, count, key_bits, s, st);
     const cudaError_t launch = cudaPeekAtLastError();
     int host = 0;
     cudaMemcpyAsync(&host, s.count, sizeof(int), cudaMemcpyDeviceToHost, st);
     const cudaError_t e = cudaStreamSynchronize(st);
-    cudaFree(base);
+    scratch.idle = e == cudaSuccess;
     const cudaError_t bad = e != cudaSuccess ? e : launch;
     if (bad != cudaSuccess) {
         cudaGetLastError();
