@@ -90,3 +90,34 @@ def test_query_sizes(pkg, gpu, oracle):
         assert np.array_equal(ga, gb) and np.array_equal(la, lb)
         box = (-2.0 - n % 5, -2, 0), (1.0 + n % 7, 3, 4)
         assert np.array_equal(a.collect_aabb(*box), b.collect_aabb(*box))
+
+
+# More than a million pairs, around a tile of 64 bodies; rays of unit length and not, from inside bodies and
+# from far away, along axes, one with a NaN and one of length zero.
+@pytest.mark.parametrize("n", [63, 64, 65, 300])
+def test_pick_tiles(pkg, gpu, oracle, n):
+    capi = pkg.capi
+    rng = np.random.default_rng(n)
+    size, pos = rng.uniform(0.3, 2.0, (n, 3)), rng.uniform(-8, 8, (n, 3))
+    q = rng.normal(size=(n, 4))
+    d = capi.make_body_descs(size, [1.0] * n, 0.5, pos, q / np.linalg.norm(q, axis=1, keepdims=True))
+    for i in range(0, n, 3):
+        d[i].shape = 1
+    rays = (1 << 20) // n + 77
+    origins = rng.uniform(-12, 12, (rays, 3)).astype(np.float32)
+    dirs = rng.normal(size=(rays, 3)).astype(np.float32)
+    dirs /= np.linalg.norm(dirs, axis=1, keepdims=True)
+    dirs[::7] = np.eye(3, dtype=np.float32)[rng.integers(0, 3, len(dirs[::7]))]
+    dirs[1::7] *= rng.uniform(0.1, 3.0, (len(dirs[1::7]), 1)).astype(np.float32)
+    origins[2::7] -= 300 * dirs[2::7]
+    origins[3::7] = pos[rng.integers(0, n, len(origins[3::7]))]
+    dirs[5], dirs[6] = 0, (np.nan, 1, 0)
+    worlds = [capi.World(api, api.default_params(), max_bodies=n) for api in (gpu, oracle)]
+    for w in worlds:
+        w.add_bodies(d)
+    (ga, la), (gb, lb) = (w.pick(origins, dirs) for w in worlds)
+    part = [worlds[0].pick(origins[i:i + 1000], dirs[i:i + 1000]) for i in range(0, rays, 1000)]  # a thread a pair
+    assert np.array_equal(ga, np.concatenate([p[0] for p in part]))
+    assert np.array_equal(la, np.concatenate([p[1] for p in part]), equal_nan=True)
+    ga[6], la[6] = gb[6], lb[6]  # which of its distances of NaN a ray takes is not the oracle's
+    assert np.array_equal(ga, gb) and np.array_equal(la, lb, equal_nan=True) and (ga >= 0).sum() > rays // 20
