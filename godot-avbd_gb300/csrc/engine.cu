@@ -1272,14 +1272,30 @@ void Engine::runSubstep(const StepParams &sp, int rounds, bool idle) {
     launchFinishBodies(d, sp, idle, stream);
 }
 
+int Engine::needRing() {
+    if (ctrRing)
+        return AVBDG_OK;
+    if (cudaMallocHost(&ctrRing, sizeof(int) * 2 * C_COUNT) != cudaSuccess) {
+        ctrRing = nullptr;
+        return fail(AVBDG_ERR_CAPACITY, "pinned counter allocation failed");
+    }
+    for (cudaEvent_t &e : ctrEvent)
+        cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
+    return AVBDG_OK;
+}
+
 int Engine::finishStep() {
-    cudaMemcpyAsync(hostCtr, d.ctr, sizeof(int) * C_COUNT, cudaMemcpyDeviceToHost, stream);
+    launches = launchCount() - launchBase;
+    const int ring = needRing();
+    if (ring)
+        return ring;
+    launchPublish(d, ctrRing, stream);
     if (cudaStreamSynchronize(stream) != cudaSuccess)
         return cudaCheck("step");
     int rc = cudaCheck("step");
     if (rc)
         return rc;
-    launches = launchCount() - launchBase;
+    std::memcpy(hostCtr, ctrRing, sizeof(int) * C_COUNT);
     return processCounters();
 }
 
@@ -1390,12 +1406,8 @@ int Engine::stepMany(int count, int substeps, int rounds) {
         const int r = rounds > 0 ? std::max(1, rounds) : std::max(2, (P.iterations + substeps - 1) / substeps);
         return planStep(1, substeps, r);
     };
-    if (!ctrRing) {
-        if (cudaMallocHost(&ctrRing, sizeof(int) * 2 * C_COUNT) != cudaSuccess)
-            return fail(AVBDG_ERR_CAPACITY, "pinned counter allocation failed");
-        for (cudaEvent_t &e : ctrEvent)
-            cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
-    }
+    if (const int ring = needRing())
+        return ring;
     int queued = -1; // ring slot of the step whose counters are not checked yet
     for (int i = 0; i < count; i++) {
         if (profiling || tuning) {
@@ -1423,7 +1435,7 @@ int Engine::stepMany(int count, int substeps, int rounds) {
             return rc;
         }
         ctrLaunches[slot] = launchCount() - launchBase;
-        cudaMemcpyAsync(ctrRing + slot * C_COUNT, d.ctr, sizeof(int) * C_COUNT, cudaMemcpyDeviceToHost, stream);
+        launchPublish(d, ctrRing + slot * C_COUNT, stream);
         cudaEventRecord(ctrEvent[slot], stream);
         if (queued >= 0) {
             rc = finishQueued(queued);

@@ -58,6 +58,7 @@ enum Counter {
     C_QDUAL,          // round-loop queue: dual tiles a round (all worlds)
     C_OLDLIVE,        // live manifolds before this step's compaction
     C_TMP,
+    C_REAP,           // a force is to be reaped (cleared by the compaction that does)
     C_COUNT
 };
 

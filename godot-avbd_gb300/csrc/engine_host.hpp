@@ -267,6 +267,7 @@ private:
     int roundsRun(int rounds) const;
     int newtonRoundsOf(int rounds) const;
     void runWorlds(const StepParams &sp, const StepPlan &plan);
+    int needRing();
     int finishStep();
     bool needGreedy() const;
 };

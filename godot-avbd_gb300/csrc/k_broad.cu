@@ -56,6 +56,13 @@ __global__ void aabbKernel(Dev d, StepParams p) {
     pdlTrigger();
     const int n = d.ctr[C_BODIES];
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
+    // The counts of the refit and of the pairs start at zero (publishKernel says why here).
+    if (g < d.NB)
+        d.nodeFlag[g] = d.pairStart[g] = 0;
+    if (g == 0) {
+        d.pairStart[d.NB] = 0;
+        d.ctr[C_PAIRSPILL] = 0;
+    }
     if (g >= n || d.meta[g].x < 0)
         return;
     f3 c, half;
@@ -511,6 +518,7 @@ __global__ void pairTotalKernel(Dev d) {
         t = d.PP;
     }
     d.ctr[C_PAIRS] = t;
+    d.ctr[C_LONG] = 0; // of the segmented sort that follows
 }
 
 // Layers and masks, not constrained, not both static (solver_broadphase.cpp:30-65 beside the bounds).
@@ -756,7 +764,6 @@ void launchRebuildTree(const Dev &d, bool multiWorld, cudaStream_t s) {
 }
 
 void launchRefit(const Dev &d, cudaStream_t s) {
-    cudaMemsetAsync(d.nodeFlag, 0, sizeof(int) * static_cast<size_t>(d.NB), s);
     ++launchCount(); launchK(refitKernel, grid(d.NB), kThreads, 0, s, d);
 }
 
@@ -766,8 +773,6 @@ bool traverseBlockFits(int block) {
 }
 
 void launchPairs(const Dev &d, int block, bool brute, cudaStream_t s) {
-    cudaMemsetAsync(d.pairStart, 0, sizeof(int) * static_cast<size_t>(d.NB + 1), s);
-    cudaMemsetAsync(d.ctr + C_PAIRSPILL, 0, sizeof(int), s);
     ++launchCount();
     if (brute)
         launchK(bruteKernel<false>, divUp(d.NB, block), block, 0, s, d);

@@ -96,11 +96,22 @@ __global__ void adjInfoKernel(Dev d) {
         adjInfoAt(d, g, e, static_cast<int>(d.adjSeq[e]));
 }
 
+__global__ void adjClearKernel(Dev d) {
+    pdlWait();
+    pdlTrigger();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i <= d.NB)
+        d.adjStart[i] = 0;
+    if (i < d.NB)
+        d.adjFill[i] = 0;
+}
+
 __global__ void adjTotalKernel(Dev d) {
     pdlWait();
     pdlTrigger();
     if (d.ctr[C_ADJ] > 2 * (d.FF + d.MM))
         atomicOr(&d.ctr[C_ERRORS], kErrAdjacency);
+    d.ctr[C_LONG] = 0; // of the segmented sort that follows
 }
 
 // ---- manifold initialize (ManifoldStore::initialize, manifold.cpp:237-435) ----
@@ -621,15 +632,16 @@ __global__ void forceInitKernel(Dev d, StepParams p) {
     const int keep = d.fBroken[f] ? 0 : 1;
     d.fKeep[f] = keep;
     if (!keep)
-        atomicOr(&d.ctr[C_TMP], 1);
+        atomicOr(&d.ctr[C_REAP], 1);
 }
 
 // Stable in-place compaction of the force list (reaping is rare; one thread walks it in order).
 __global__ void forceCompactKernel(Dev d) {
     pdlWait();
     pdlTrigger();
-    if (!d.ctr[C_TMP])
+    if (!d.ctr[C_REAP])
         return;
+    d.ctr[C_REAP] = 0;
     const int nf = d.ctr[C_FORCES];
     int w = 0;
     for (int f = 0; f < nf; f++) {
@@ -673,8 +685,7 @@ void prepareNarrowPhase() {
 }
 
 void launchAdjacency(const Dev &d, cudaStream_t s) {
-    cudaMemsetAsync(d.adjStart, 0, sizeof(int) * static_cast<size_t>(d.NB + 1), s);
-    cudaMemsetAsync(d.adjFill, 0, sizeof(int) * static_cast<size_t>(d.NB), s);
+    ++launchCount(); launchK(adjClearKernel, grid(d.NB + 1), kThreads, 0, s, d);
     ++launchCount(); launchK(adjCountKernel, grid(d.FF + d.MM), kThreads, 0, s, d);
     // Slots past the last body count zero, so scanning the whole capacity gives the same starts.
     scanExclusive(d.adjStart, d.adjStart, d.NB + 1, nullptr, d.ctr + C_ADJ, d.scanScratch, s);
@@ -780,7 +791,6 @@ void launchRebase(const Dev &d, const StepParams &p, cudaStream_t s) {
 void launchForceInit(const Dev &d, const StepParams &p, bool forces, cudaStream_t s) {
     if (!forces)
         return;
-    cudaMemsetAsync(d.ctr + C_TMP, 0, sizeof(int), s);
     ++launchCount(); launchK(forceInitKernel, grid(d.FF), kThreads, 0, s, d, p);
     ++launchCount(); launchK(forceCompactKernel, 1, 1, 0, s, d);
 }

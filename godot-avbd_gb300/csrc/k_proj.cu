@@ -345,7 +345,6 @@ int brakeGridBlocks() {
 }
 
 void launchProjActive(const Dev &d, cudaStream_t s) {
-    cudaMemsetAsync(d.wActive, 0, sizeof(int) * static_cast<size_t>(d.WW), s);
     ++launchCount(); launchK(projActiveKernel, residentGrid(projActiveKernel, kThreads, grid(d.MM)), kThreads, 0, s, d);
     scanExclusive(d.mActive, d.pairValid, d.MM, d.ctr + C_LIVE, d.ctr + C_SPECN, d.scanScratch, s);
     ++launchCount(); launchK(specScatterKernel, residentGrid(specScatterKernel, kThreads, grid(d.MM)), kThreads, 0, s, d, d.mActive, d.pairValid);

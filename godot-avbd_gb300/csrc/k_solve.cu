@@ -249,6 +249,18 @@ __global__ void finishKernel(Dev d, StepParams p, int idle) {
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g < n && d.meta[g].x >= 0)
         finishAt(d, p, g, idle);
+    if (g < d.WW)
+        d.wActive[g] = 0; // until the projection finds manifolds to move
+}
+
+// The counters to the host's memory. As a kernel behind the step's others it starts when they end; a copy,
+// like a memset between kernels, costs the work around it some microseconds of order (publish: 13 us a step;
+// each memset 5-8), which is why the kernels of a step clear each other's counts.
+__global__ void publishKernel(const int *ctr, int *to, int n) {
+    pdlWait();
+    pdlTrigger();
+    if (threadIdx.x < n)
+        to[threadIdx.x] = ctr[threadIdx.x];
 }
 
 // ---- update set and colouring (solver_solve.cpp:263-424) ----
@@ -257,6 +269,10 @@ __global__ void contactOnlyInitKernel(Dev d) {
     pdlWait();
     pdlTrigger();
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
+    if (g < d.WW)
+        d.wColour[g] = 0;
+    if (g <= kMaxColours)
+        d.colourCount[g] = 0;
     if (g >= d.ctr[C_BODIES])
         return;
     const bool dyn = d.meta[g].x >= 0 && d.x[g].w > 0.0f, update = selectBody(d, g, dyn);
@@ -375,8 +391,8 @@ static int grid(int n) { return divUp(n > 0 ? n : 1, kThreads); }
 static int queueGridMax();
 
 void launchContactOnly(const Dev &d, cudaStream_t s) {
-    cudaMemsetAsync(d.wColour, 0, sizeof(int) * static_cast<size_t>(d.WW), s);
-    ++launchCount(); launchK(contactOnlyInitKernel, grid(d.NB), kThreads, 0, s, d);
+    const int most = d.NB > d.WW ? d.NB : d.WW;
+    ++launchCount(); launchK(contactOnlyInitKernel, grid(most > kMaxColours ? most : kMaxColours + 1), kThreads, 0, s, d);
     ++launchCount(); launchK(contactOnlyMarkKernel, grid(d.FF), kThreads, 0, s, d);
 }
 
@@ -445,7 +461,6 @@ void launchColour(const Dev &d, bool needGreedy, bool everyWorld, cudaStream_t s
 }
 
 void launchColourLists(const Dev &d, int contactOnlyOverflow, cudaStream_t s) {
-    cudaMemsetAsync(d.colourCount, 0, sizeof(int) * (kMaxColours + 1), s);
     ++launchCount(); launchK(colourListKernel, grid(d.NB), kThreads, 0, s, d, contactOnlyOverflow);
 }
 
@@ -454,7 +469,12 @@ void launchWarmstartBodies(const Dev &d, const StepParams &p, cudaStream_t s) {
 }
 
 void launchFinishBodies(const Dev &d, const StepParams &p, bool idle, cudaStream_t s) {
-    ++launchCount(); launchK(finishKernel, grid(d.NB), kThreads, 0, s, d, p, idle ? 1 : 0);
+    ++launchCount(); launchK(finishKernel, grid(d.NB > d.WW ? d.NB : d.WW), kThreads, 0, s, d, p, idle ? 1 : 0);
+}
+
+void launchPublish(const Dev &d, int *to, cudaStream_t s) {
+    static_assert(C_COUNT <= kThreads, "one block");
+    ++launchCount(); launchK(publishKernel, 1, kThreads, 0, s, d.ctr, to, static_cast<int>(C_COUNT));
 }
 
 void launchStamps(const Dev &d, const StepParams &p, bool mixedOnly, cudaStream_t s) {

@@ -65,6 +65,7 @@ void launchColourLists(const Dev &d, int contactOnlyOverflow, cudaStream_t s);
 // ---- substep (k_solve.cu) ----
 void launchWarmstartBodies(const Dev &d, const StepParams &p, cudaStream_t s);
 // BDF1 velocities; with `idle` (the tick's last substep) also idle detection for sleeping.
+void launchPublish(const Dev &d, int *to, cudaStream_t s); // the counters, to pinned memory
 void launchFinishBodies(const Dev &d, const StepParams &p, bool idle, cudaStream_t s);
 // Stamps (precompute) of manifolds touching the overflow set; `mixedOnly` restricts to those that
 // also touch a coloured body (recomputed after the colour passes).

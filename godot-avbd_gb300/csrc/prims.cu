@@ -566,7 +566,6 @@ void uniqueSorted(const uint64_t *keys, int n, uint64_t *out, int *d_count, void
 template <typename T>
 static void segmentedSort(T *data, const int *start, int segCapacity, const int *d_segments, int *longList,
                           int *longCount, T *tmp, cudaStream_t stream) {
-    cudaMemsetAsync(longCount, 0, sizeof(int), stream);
     const int grid = divUp(segCapacity > 0 ? segCapacity : 1, 256);
     ++launchCount(); launchK(segSmallKernel<T>, grid < 4096 ? grid : 4096, 256, 0, stream, data, start, segCapacity, d_segments, longList,
                                                                    longCount);

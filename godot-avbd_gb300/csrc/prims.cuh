@@ -74,7 +74,7 @@ void radixSortPairs(uint64_t *keys, uint32_t *values, uint64_t *keysAlt, uint32_
 // Sorts each segment data[start[s] .. start[s+1]) ascending, for s < *d_segments. Segments up to 32
 // entries are sorted by one thread, up to 8192 by one block in shared memory, longer ones by a
 // tiled rank sort over several blocks through `tmp` (same capacity as `data`). Values must be
-// distinct within a segment. `longList` needs `segCapacity` ints, `longCount` one int.
+// distinct within a segment. `longList` needs `segCapacity` ints, `longCount` one int, zero before.
 void segmentedSortU32(uint32_t *data, uint32_t *tmp, const int *start, int segCapacity, const int *d_segments,
                       int *longList, int *longCount, cudaStream_t stream);
 void segmentedSortU64(uint64_t *data, uint64_t *tmp, const int *start, int segCapacity, const int *d_segments,
