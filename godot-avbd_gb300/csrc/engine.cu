@@ -250,8 +250,6 @@ Engine::Engine(const avbdg_params &params, int maxBodies, int maxForces, int max
         tuned = tunedBase;
     }
     cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking);
-    for (auto &e : ev)
-        cudaEventCreate(&e);
     armStore = P.jacobian_rebuild_distance > 0.0f;
     const int nb = std::max(maxBodies, 64);
     allocate(nb, std::max(1024, 8 * nb), std::max(maxForces, 16), std::max(4096, 16 * nb), std::max(maxWorlds, 1));
@@ -272,9 +270,6 @@ Engine::~Engine() {
             cudaEventDestroy(e);
     for (cudaEvent_t e : evPool)
         cudaEventDestroy(e);
-    for (auto &e : ev)
-        if (e)
-            cudaEventDestroy(e);
     if (stream)
         cudaStreamDestroy(stream);
 }
@@ -958,19 +953,23 @@ void Engine::recordPhase(cudaEvent_t e) {
 int Engine::broadPhase(const StepParams &sp, const StepPlan &plan) {
     if (plan.adjAtStart)
         launchAdjacency(d, stream);
+    startPhase(0);
     if (plan.front) {
         if (plan.rebuild) { // the tree's codes and order are dumped on the reference's schedule
             launchAabb(d, sp, stream);
+            startPhase(kNoPhase);
             launchRebuildTree(d, plan.multiWorld, stream);
         }
         beginSpan();
         launchWorldPairs(d, sp, plan.front, stream);
+        startPhase(kNoPhase);
         endSpan(kTraverse);
         if (sp.sleepFrames > 0)
             launchSleepWakePairs(d, stream);
         return AVBDG_OK;
     }
     launchAabb(d, sp, stream);
+    startPhase(kNoPhase);
     if (!plan.anyTree) {
         cudaMemsetAsync(d.ctr + C_PAIRS, 0, sizeof(int), stream);
         cudaMemcpyAsync(d.ctr + C_CAND, d.ctr + C_LIVE, sizeof(int), cudaMemcpyDeviceToDevice, stream);
@@ -1002,25 +1001,22 @@ bool Engine::enqueueStep(const StepPlan &plan) {
     if (plan.mode == 0) {
         const StepParams sp = stepParams(P.dt);
         broadPhase(sp, plan);
-        recordPhase(ev[1]);
         if (!launchesOk())
             return false;
         warmstartAndSelect(sp, plan);
         if (plan.worldCount) {
-            recordPhase(ev[2]);
             if (launchesOk())
                 runWorlds(sp, plan);
-            recordPhase(ev[3]);
             return launchesOk();
         }
         projectContacts(sp, false, 0.0f);
-        recordPhase(ev[2]);
         if (!launchesOk())
             return false;
+        startPhase(2);
         runSubstep(sp, P.iterations, true);
-        recordPhase(ev[3]);
         if (!launchesOk())
             return false;
+        startPhase(3);
         projectContacts(sp, P.position_projection != 0, 0.0f);
         launchRebase(d, sp, stream);
         return launchesOk();
@@ -1028,17 +1024,15 @@ bool Engine::enqueueStep(const StepPlan &plan) {
     const int substeps = plan.substeps;
     const StepParams sp = stepParams(P.dt * static_cast<real>(substeps));
     broadPhase(sp, plan);
-    recordPhase(ev[1]);
     if (!launchesOk())
         return false;
     warmstartAndSelect(sp, plan);
-    recordPhase(ev[2]);
     if (plan.worldCount) {
         if (launchesOk())
             runWorlds(sp, plan);
-        recordPhase(ev[3]);
         return launchesOk();
     }
+    startPhase(2);
     for (int sub = 0; sub < substeps; ++sub) {
         if (!launchesOk())
             return false;
@@ -1047,9 +1041,9 @@ bool Engine::enqueueStep(const StepPlan &plan) {
         projectContacts(sp, false, P.dt * static_cast<real>(substeps - sub));
         runSubstep(sp, plan.rounds, sub + 1 == substeps);
     }
-    recordPhase(ev[3]);
     if (!launchesOk())
         return false;
+    startPhase(3);
     projectContacts(sp, P.position_projection != 0, sp.collisionDt);
     launchRebase(d, sp, stream);
     return launchesOk();
@@ -1082,9 +1076,6 @@ int Engine::enqueuePlan(const StepPlan &plan) {
     launchBase = launchCount();
     graphSpans = nullptr;
     lastGraph = false;
-    // The step's device time starts when its work is handed to the stream: after a capture and
-    // instantiation (host work the device only waits for), before an eager enqueue or a launch.
-    const auto startClock = [&] { cudaEventRecord(ev[0], stream); };
     const bool trial = tuning && tuneTrial >= 0;
     if (trial)
         configureTrial();
@@ -1096,7 +1087,6 @@ int Engine::enqueuePlan(const StepPlan &plan) {
         // counts are read on the device, so adding or removing worlds keeps the cache.
         const bool capture = it == graphs.end() && planSeen[k]++ > 0;
         if (it == graphs.end() && !capture) {
-            startClock();
             if (!enqueueStep(plan))
                 return launchFailure();
         } else if (it == graphs.end()) {
@@ -1131,8 +1121,7 @@ int Engine::enqueuePlan(const StepPlan &plan) {
                     cudaEventDestroy(s.b);
                 }
                 spans.clear();
-                startClock();
-                if (!enqueueStep(plan))
+                    if (!enqueueStep(plan))
                     return launchFailure();
             } else {
                 Graph gr{exec, launchCount() - before, {}};
@@ -1141,18 +1130,15 @@ int Engine::enqueuePlan(const StepPlan &plan) {
             }
         }
         if (it != graphs.end()) {
-            startClock();
             cudaGraphLaunch(it->second.exec, stream);
             launchBase = launchCount() - it->second.launches; // kernels inside the graph
             graphSpans = &it->second.spans;
             lastGraph = true;
         }
     } else {
-        startClock();
         if (!enqueueStep(plan))
             return launchFailure();
     }
-    cudaEventRecord(ev[4], stream);
     timed = true;
     return AVBDG_OK;
 }
@@ -1164,17 +1150,22 @@ int Engine::runPlan(const StepPlan &plan) {
 
 // warmstartForces + selectUpdateBodies (solver_solve.cpp:31-105, 263-424).
 int Engine::warmstartAndSelect(const StepParams &sp, const StepPlan &plan) {
+    startPhase(1);
     launchForceInit(d, sp, nForces > 0, stream);
+    if (nForces > 0)
+        startPhase(kNoPhase);
     if (plan.front) {
         const bool select = sp.sleepFrames == 0 && !needGreedy();
         beginSpan();
         launchWorldContacts(d, sp, nRound > 0, select, plan.front, stream);
+        startPhase(kNoPhase);
         endSpan(kNarrow);
         if (select)
             return AVBDG_OK;
     } else {
         beginSpan();
         launchManifoldInit(d, sp, nRound > 0, tuned.narrow, stream);
+        startPhase(kNoPhase);
         endSpan(kNarrow);
         launchManifoldCompact(d, plan.worldMajor, stream);
         launchAdjacency(d, stream);
@@ -1190,6 +1181,7 @@ int Engine::warmstartAndSelect(const StepParams &sp, const StepPlan &plan) {
 // Solver::projectContacts (solver_projection.cpp:67-281).
 void Engine::projectContacts(const StepParams &sp, bool positions, real window) {
     launchProjActive(d, stream);
+    startPhase(kNoPhase);
     if (sp.specMargin > 0.0f)
         launchBrake(d, window > 0.0f ? window : sp.collisionDt, stream);
     if (positions && sp.projIters > 0)
@@ -1221,12 +1213,15 @@ void Engine::runWorlds(const StepParams &sp, const StepPlan &plan) {
     run.project = P.position_projection != 0 && sp.projIters > 0;
     run.colours = needGreedy();
     run.multiWorld = plan.multiWorld;
+    startPhase(2);
     launchWorlds(d, sp, run, plan.worldCount, plan.worldBodies, stream);
+    startPhase(kNoPhase);
 }
 
 // Solver::runSubstep + iterateBody (solver_step.cpp:79-105, 195-316).
 void Engine::runSubstep(const StepParams &sp, int rounds, bool idle) {
     launchWarmstartBodies(d, sp, stream);
+    startPhase(kNoPhase);
     const int newtonRounds = newtonRoundsOf(rounds);
     const bool colours = needGreedy();
     const bool inPlace = nForces == 0;
@@ -2003,9 +1998,13 @@ int Engine::stats(avbdg_stats &out) {
         out.block_traverse = tuned.traverse;
     }
     if (timed) {
-        float t[4] = {};
+        unsigned long long at[5];
+        std::memcpy(at, hostCtr + C_CLOCK, sizeof(at));
+        if (at[3] < at[2]) // a step whose finish is part of its solve
+            at[3] = at[4];
+        double t[4];
         for (int i = 0; i < 4; i++)
-            cudaEventElapsedTime(&t[i], ev[i], ev[i + 1]);
+            t[i] = at[i + 1] > at[i] ? static_cast<double>(at[i + 1] - at[i]) * 1.0e-6 : 0.0;
         out.broad_ms = t[0];
         out.graph_ms = t[1];
         out.solve_ms = t[2];

@@ -59,7 +59,9 @@ enum Counter {
     C_OLDLIVE,        // live manifolds before this step's compaction
     C_TMP,
     C_REAP,           // a force is to be reaped (cleared by the compaction that does)
-    C_COUNT
+    C_LAST,
+    C_CLOCK = (C_LAST + 1) / 2 * 2, // five 64-bit times (ns): the starts of a step's phases, its end
+    C_COUNT = C_CLOCK + 10
 };
 
 constexpr int kErrPairs = 1;
@@ -103,6 +105,7 @@ struct ManifoldBuf {
 struct Dev {
     int NB, MM, FF, PP, WW; // capacities
     int ARM;                // 1: the arm-cache arrays of ManifoldBuf are allocated
+    int stamp;              // k + 1: the launch is the first of the step's phase k (stampPhase); 0: not
     long long waitLimit;    // spins a dataflow wait makes before it reports a timeout
     unsigned *gridBar;      // grid barrier of the cooperative sweeps: arrivals, generation
     // Round-loop tile queue (k_queue.cu): each world's live manifolds grouped together (wManStart,
@@ -192,6 +195,17 @@ __device__ __forceinline__ int bodyWorld(const Dev &d, int g) { return d.meta[g]
 // Contact slot c of manifold m. The contact arrays are slot-major (MM entries per slot), so a warp
 // reading slot c of 32 consecutive manifolds reads 512 contiguous bytes.
 AVBD_HD int cslot(const Dev &d, int m, int c) { return c * d.MM + m; }
+__device__ __forceinline__ unsigned long long nowNs() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+// The start of a phase of the step, by its first kernel (an event between two kernels of a captured step
+// keeps them 8 us apart).
+__device__ __forceinline__ void stampPhase(const Dev &d) {
+    if (d.stamp > 0 && blockIdx.x == 0 && threadIdx.x == 0)
+        reinterpret_cast<unsigned long long *>(d.ctr + C_CLOCK)[d.stamp - 1] = nowNs();
+}
 // List position of body g: the world's bodies in list order (reverse creation) occupy
 // [wBase, wBase + wCount).
 __device__ __forceinline__ int listPos(const Dev &d, int g) {

@@ -157,7 +157,6 @@ private:
     int finishQueued(int slot);
     bool roomy() const;
     int colourSizes[kMaxColours + 1] = {};
-    cudaEvent_t ev[5] = {};
     bool timed = false;
     std::string err;
     // Profiling: event pairs around the hot launches of the current step.
@@ -259,6 +258,9 @@ private:
     int runPlan(const StepPlan &plan);
     void dropGraphs();
     void recordPhase(cudaEvent_t e);
+    // The next launch that can stamps the start of phase k (broad, graph, solve, finish).
+    static constexpr int kNoPhase = -1;
+    void startPhase(int k) { d.stamp = k + 1; }
     int broadPhase(const StepParams &sp, const StepPlan &plan);
     int warmstartAndSelect(const StepParams &sp, const StepPlan &plan);
     void sortLiveByWorld();

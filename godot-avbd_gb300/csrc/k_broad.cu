@@ -54,6 +54,7 @@ __device__ __forceinline__ void sweptBox(const Dev &d, const StepParams &p, int 
 __global__ void aabbKernel(Dev d, StepParams p) {
     pdlWait();
     pdlTrigger();
+    stampPhase(d);
     const int n = d.ctr[C_BODIES];
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     // The counts of the refit and of the pairs start at zero (publishKernel says why here).
@@ -613,6 +614,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
         worldPairsKernel(const __grid_constant__ Dev d, const __grid_constant__ StepParams p) {
     pdlWait();
     pdlTrigger();
+    stampPhase(d);
     extern __shared__ __align__(32) unsigned char smem[];
     __shared__ int warpSums[kPairThreads / 32];
     Box *box = reinterpret_cast<Box *>(smem);

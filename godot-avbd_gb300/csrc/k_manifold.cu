@@ -329,6 +329,7 @@ template <bool ROUND>
 __global__ void manifoldInitKernel(Dev d, StepParams p) {
     pdlWait();
     pdlTrigger();
+    stampPhase(d);
     const int n = d.ctr[C_CAND];
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         manifoldInitAt<ROUND>(d, p, i);
@@ -409,6 +410,7 @@ __global__ void __launch_bounds__(kContactThreads, 1)
         worldContactsKernel(const __grid_constant__ Dev d, const __grid_constant__ StepParams p, int select) {
     pdlWait();
     pdlTrigger();
+    stampPhase(d);
     __shared__ int warpSums[kContactThreads / 32], ranks[kContactThreads], longCount;
     const int rank = clusterRank(), size = clusterSize(), lane = threadIdx.x & 31;
     // Threads over the cluster a warp at a time, so that few items still spread over its SMs.
@@ -611,6 +613,7 @@ __device__ __forceinline__ f3 warmPenalty(f3 k, real gamma, real stiffness) {
 __global__ void forceInitKernel(Dev d, StepParams p) {
     pdlWait();
     pdlTrigger();
+    stampPhase(d);
     const int f = blockIdx.x * blockDim.x + threadIdx.x;
     const int nf = d.ctr[C_FORCES];
     if (f >= nf)

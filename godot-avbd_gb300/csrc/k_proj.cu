@@ -33,6 +33,7 @@ constexpr int kBrakeThreads = 512;
 __global__ void projActiveKernel(Dev d) {
     pdlWait();
     pdlTrigger();
+    stampPhase(d);
     const int n = d.ctr[C_LIVE];
     for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < n; m += gridDim.x * blockDim.x)
         projActiveAt(d, m);

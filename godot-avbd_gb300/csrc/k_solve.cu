@@ -236,6 +236,7 @@ __global__ void overflowApplyKernel(Dev d, StepParams p) {
 __global__ void warmstartKernel(Dev d, StepParams p) {
     pdlWait();
     pdlTrigger();
+    stampPhase(d);
     const int n = d.ctr[C_BODIES];
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g < n && d.meta[g].x >= 0)
@@ -256,11 +257,18 @@ __global__ void finishKernel(Dev d, StepParams p, int idle) {
 // The counters to the host's memory. As a kernel behind the step's others it starts when they end; a copy,
 // like a memset between kernels, costs the work around it some microseconds of order (publish: 13 us a step;
 // each memset 5-8), which is why the kernels of a step clear each other's counts.
-__global__ void publishKernel(const int *ctr, int *to, int n) {
+__global__ void publishKernel(const int *ctr, int *to) {
     pdlWait();
     pdlTrigger();
-    if (threadIdx.x < n)
-        to[threadIdx.x] = ctr[threadIdx.x];
+    __shared__ unsigned long long end;
+    if (threadIdx.x == 0)
+        end = nowNs();
+    __syncthreads();
+    const int i = threadIdx.x;
+    if (i < C_CLOCK + 8)
+        to[i] = ctr[i];
+    else if (i < C_COUNT)
+        to[i] = reinterpret_cast<const int *>(&end)[i - C_CLOCK - 8];
 }
 
 // ---- update set and colouring (solver_solve.cpp:263-424) ----
@@ -474,7 +482,7 @@ void launchFinishBodies(const Dev &d, const StepParams &p, bool idle, cudaStream
 
 void launchPublish(const Dev &d, int *to, cudaStream_t s) {
     static_assert(C_COUNT <= kThreads, "one block");
-    ++launchCount(); launchK(publishKernel, 1, kThreads, 0, s, d.ctr, to, static_cast<int>(C_COUNT));
+    ++launchCount(); launchK(publishKernel, 1, kThreads, 0, s, d.ctr, to);
 }
 
 void launchStamps(const Dev &d, const StepParams &p, bool mixedOnly, cudaStream_t s) {

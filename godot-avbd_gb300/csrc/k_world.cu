@@ -1856,6 +1856,7 @@ __global__ void __launch_bounds__(kMaxWorldThreads, 1)
         worldKernel(const __grid_constant__ Dev d, const __grid_constant__ StepParams p, const __grid_constant__ WorldRun r) {
     pdlWait();
     pdlTrigger();
+    stampPhase(d);
     extern __shared__ __align__(32) unsigned char smem[];
     __shared__ int shared[4], deepest[2];
     __shared__ real carry[32];
