@@ -88,3 +88,23 @@ def test_batch_state_all_round_trip(pkg, gpu, io_path):
     assert e.value.code == capi.ERR_NONFINITE
     assert _equal(batch.state_all(), after)
     batch.close()
+
+
+# Either side of the size from which the fields are copied (8192 bodies): parts of a state, written and read
+# in any range, and refusals.
+@pytest.mark.parametrize("n", [1, 8191, 8192, 8193, 9000])
+def test_state_at_the_copied_size(pkg, gpu, io_path, n):
+    capi, rng = pkg.capi, np.random.default_rng(n)
+    pos = np.stack([np.arange(n) * 3.0, np.zeros(n), np.zeros(n)], 1)
+    w = capi.World(gpu, gpu.default_params(), max_bodies=n)
+    w.add_bodies(capi.make_body_descs([[1, 1, 1]] * n, [1.0] * n, 0.5, pos))
+    want = [a.copy() for a in w.state()]
+    for k, field in enumerate(("position", "orientation", "velocity", "angular_velocity")):
+        want[k] = rng.normal(size=want[k].shape).astype(np.float32)
+        w.set_state(**{field: want[k]})
+        assert _equal(w.state(), want)
+    bad = want[2].copy()
+    bad[n - 1, 2] = np.nan
+    with pytest.raises(capi.AvbdError) as e:
+        w.set_state(position=want[0] + 1, velocity=bad)
+    assert e.value.code == capi.ERR_NONFINITE and _equal(w.state(), want)
