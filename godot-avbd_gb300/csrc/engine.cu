@@ -910,6 +910,9 @@ Engine::StepPlan Engine::planStep(int mode, int substeps, int rounds) {
             plan.worldBodies = bodies;
         }
     }
+    if (plan.greedy && worldAllowed && most <= colourWorldMost())
+        for (plan.colourMost = 64; plan.colourMost < most;)
+            plan.colourMost *= 2;
     if (worldAllowed && worlds() == 1 && plan.anyTree && most <= worldPairsMost())
         plan.front = most;
     return plan;
@@ -937,9 +940,9 @@ void Engine::sortLiveByWorld() {
 
 std::string Engine::StepPlan::key() const {
     char buf[128];
-    std::snprintf(buf, sizeof(buf), "%d/%d/%d/%d%d%d%d%d%d%d%d%d/%d/%d/%d", mode, substeps, rounds, adjAtStart ? 1 : 0,
+    std::snprintf(buf, sizeof(buf), "%d/%d/%d/%d%d%d%d%d%d%d%d%d/%d/%d/%d/%d", mode, substeps, rounds, adjAtStart ? 1 : 0,
                   anyTree ? 1 : 0, rebuild ? 1 : 0, forces ? 1 : 0, greedy ? 1 : 0, multiWorld ? 1 : 0,
-                  round ? 1 : 0, brute ? 1 : 0, worldMajor ? 1 : 0, worldCount, worldBodies, front);
+                  round ? 1 : 0, brute ? 1 : 0, worldMajor ? 1 : 0, worldCount, worldBodies, front, colourMost);
     return buf;
 }
 
@@ -1173,7 +1176,7 @@ int Engine::warmstartAndSelect(const StepParams &sp, const StepPlan &plan) {
     if (sp.sleepFrames > 0)
         launchSleepSelect(d, sp, stream);
     launchContactOnly(d, stream);
-    launchColour(d, needGreedy(), !P.contact_only_overflow, stream);
+    launchColour(d, needGreedy(), !P.contact_only_overflow, plan.colourMost, stream);
     launchColourLists(d, P.contact_only_overflow, stream);
     return AVBDG_OK;
 }

@@ -238,6 +238,7 @@ private:
         // bodies, each rounded up to a power of two (0: separate launches).
         int worldCount = 0, worldBodies = 0;
         int front = 0; // the step's first half as two launches of one cluster: the world's bodies (0: separate)
+        int colourMost = 0; // colouring by a block a world, of up to this many bodies (0: across the store)
         bool worldMajor = false; // the compaction leaves the live manifolds in world order
         std::string key() const;
     };

@@ -58,7 +58,9 @@ void launchForceInit(const Dev &d, const StepParams &p, bool forces, cudaStream_
 void launchContactOnly(const Dev &d, cudaStream_t s);
 // Greedy colouring of dynamic bodies in list order (when `needGreedy`), colours in d.colour;
 // unless `everyWorld`, only worlds a force touches are coloured (the rest go to overflow).
-void launchColour(const Dev &d, bool needGreedy, bool everyWorld, cudaStream_t s);
+// `largest`: at least the bodies of the store's largest world, if at most colourWorldMost(); else 0.
+int colourWorldMost();
+void launchColour(const Dev &d, bool needGreedy, bool everyWorld, int largest, cudaStream_t s);
 // Contact-only bodies to the overflow colour, then per-colour body lists and counts.
 void launchColourLists(const Dev &d, int contactOnlyOverflow, cudaStream_t s);
 

@@ -179,3 +179,16 @@ def test_forces_as_separate_launches(pkg, gpu, monkeypatch, n, params, interleav
     here = run_forces(gpu, capi, world, params, interleaved=interleaved)
     monkeypatch.setenv("AVBDG_NO_WORLD", "1")
     assert same(here, run_forces(gpu, capi, world, params, interleaved=interleaved))
+
+
+# The colouring by a block a world: more bodies than its threads, every body coloured or those with forces,
+# the same bits as across the store.
+@pytest.mark.parametrize("params", [{}, {"contact_only_overflow": 0}])
+@pytest.mark.parametrize("n", [1025, 2600])
+def test_colouring(pkg, gpu, monkeypatch, n, params):
+    capi = pkg.capi
+    d, forces = tangle(capi, n, n)
+    world = d, forces[:60] + forces[-40:]
+    here = run_forces(gpu, capi, world, params, steps=8)
+    monkeypatch.setenv("AVBDG_NO_WORLD", "1")
+    assert same(here, run_forces(gpu, capi, world, params, steps=8))
