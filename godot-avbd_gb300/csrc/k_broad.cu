@@ -601,9 +601,11 @@ __global__ void candTotalKernel(Dev d) {
 //
 // For a store of one world of up to some thousand bodies the separate launches (bounds, pair counts, a
 // scan, pairs, their sort, filter, a scan, acquisition) are ~20 fixed costs of a few microseconds. Here a
-// cluster does them all: every CTA holds the world's boxes in shared memory, a warp tests one body
-// against the bodies before it in slots, 32 at a time in list order, so its partners come out sorted;
-// counts are scanned by every CTA reading all of them (clusterShare).
+// cluster does them all: every CTA holds the world's boxes in shared memory, a warp tests two bodies
+// against the bodies before them in slots, 32 at a time in list order, so their partners come out sorted;
+// counts are scanned by every CTA reading all of them (clusterShare). The filter and the acquisition are
+// chains of loads for a handful of pairs a body: eight lanes take a body
+// (a warp each and one body a test: 69 us for a lattice of 2431 boxes, 44 for a pile of 1653; now 43 and 31).
 constexpr int kPairThreads = 512;
 
 struct Box {
@@ -651,15 +653,38 @@ __global__ void __launch_bounds__(kPairThreads, 1)
         return found;
     };
     int *counts = d.pairSpill, *valid = d.solveFail; // scratch per list position
-    for (int g = warp; g < n; g += warps) {
-        const int lp = n - 1 - g;
-        int *stash = d.pairStash + static_cast<size_t>(lp) * kPairStash;
-        const int found = partners(g, [&](bool hit, int at, int b) {
-            if (hit && at < kPairStash)
-                stash[at] = b;
-        });
-        if (lane == 0)
-            counts[lp] = found;
+    for (int t = warp; 2 * t < n; t += warps) {
+        const int g = 2 * t; // and the next
+        const bool two = g + 1 < n;
+        const real4 lo0 = box[g].lo, hi0 = box[g].hi, lo1 = box[two ? g + 1 : g].lo, hi1 = box[two ? g + 1 : g].hi;
+        int *stash0 = d.pairStash + static_cast<size_t>(n - 1 - g) * kPairStash, *stash1 = stash0 - kPairStash;
+        int found0 = 0, found1 = 0;
+        for (int b0 = g; b0 >= 0; b0 -= 32) {
+            const int b = b0 - lane;
+            bool hit0 = false, hit1 = false;
+            if (b >= 0) {
+                const real4 bl = box[b].lo, bh = box[b].hi;
+                const f3 l{bl.x, bl.y, bl.z}, h{bh.x, bh.y, bh.z};
+                hit0 = b < g && overlapClosed(f3{lo0.x, lo0.y, lo0.z}, f3{hi0.x, hi0.y, hi0.z}, l, h);
+                hit1 = two && overlapClosed(f3{lo1.x, lo1.y, lo1.z}, f3{hi1.x, hi1.y, hi1.z}, l, h);
+            }
+            const unsigned hits0 = __ballot_sync(0xffffffffu, hit0), hits1 = __ballot_sync(0xffffffffu, hit1);
+            if ((hits0 | hits1) == 0)
+                continue;
+            const unsigned below = (1u << lane) - 1u;
+            const int at0 = found0 + __popc(hits0 & below), at1 = found1 + __popc(hits1 & below);
+            if (hit0 && at0 < kPairStash)
+                stash0[at0] = b;
+            if (hit1 && at1 < kPairStash)
+                stash1[at1] = b;
+            found0 += __popc(hits0);
+            found1 += __popc(hits1);
+        }
+        if (lane == 0) {
+            counts[n - 1 - g] = found0;
+            if (two)
+                counts[n - 2 - g] = found1;
+        }
     }
     clusterSync(size);
     // Pairs in key order: this CTA's list positions, a warp each; the filter on the way.
@@ -673,26 +698,36 @@ __global__ void __launch_bounds__(kPairThreads, 1)
         run += all;
     }
     __syncthreads();
-    for (int lp = share.lo + static_cast<int>(threadIdx.x >> 5); lp < share.hi; lp += kPairThreads / 32) {
-        const int g = n - 1 - lp, start = d.pairStart[lp], found = counts[lp];
+    const int part = lane >> 3, eighth = lane & 7; // eight lanes a list position
+    const auto emit = [&](bool on, int lp, int start, int at, int b) {
+        if (!on || start + at >= d.PP)
+            return false;
+        d.pairs[start + at] = (static_cast<uint64_t>(lp) << 32) | static_cast<uint32_t>(n - 1 - b);
+        const bool ok = pairAllowed(d, n - 1 - lp, b);
+        d.pairValid[start + at] = ok ? 1 : 0;
+        return ok;
+    };
+    for (int lp0 = share.lo + 4 * static_cast<int>(threadIdx.x >> 5); lp0 < share.hi; lp0 += 4 * (kPairThreads / 32)) {
+        const int lp = lp0 + part, found = lp < share.hi ? counts[lp] : 0, start = lp < share.hi ? d.pairStart[lp] : 0;
+        const bool stashed = found <= kPairStash;
+        const int *stash = d.pairStash + static_cast<size_t>(lp) * kPairStash;
+        const int most = __reduce_max_sync(0xffffffffu, stashed ? found : 0);
         int allowed = 0;
-        const auto emit = [&](bool on, int at, int b) {
-            bool ok = false;
-            if (on && start + at < d.PP) {
-                d.pairs[start + at] = (static_cast<uint64_t>(lp) << 32) | static_cast<uint32_t>(n - 1 - b);
-                ok = pairAllowed(d, g, b);
-                d.pairValid[start + at] = ok ? 1 : 0;
-            }
-            allowed += __popc(__ballot_sync(0xffffffffu, ok));
-        };
-        if (found <= kPairStash) {
-            const int *stash = d.pairStash + static_cast<size_t>(lp) * kPairStash;
-            for (int at = lane; at - lane < found; at += 32)
-                emit(at < found, at, at < found ? stash[at] : 0);
-        } else {
-            partners(g, emit);
+        for (int at = eighth; at - eighth < most; at += 8) {
+            const bool on = stashed && at < found;
+            const bool ok = emit(on, lp, start, at, on ? stash[at] : 0);
+            allowed += __popc(__ballot_sync(0xffffffffu, ok) >> (8 * part) & 0xffu);
         }
-        if (lane == 0)
+        for (unsigned open = __ballot_sync(0xffffffffu, !stashed && eighth == 0); open; open &= open - 1) { // the rare rest
+            const int from = __ffs(open) - 1, l = lp0 + (from >> 3), s0 = __shfl_sync(0xffffffffu, start, from);
+            int all = 0;
+            partners(n - 1 - l, [&](bool hit, int at, int b) {
+                all += __popc(__ballot_sync(0xffffffffu, emit(hit, l, s0, at, b)));
+            });
+            if (lane >> 3 == from >> 3)
+                allowed = all;
+        }
+        if (eighth == 0 && lp < share.hi)
             valid[lp] = allowed;
     }
     clusterSync(size);
@@ -709,14 +744,17 @@ __global__ void __launch_bounds__(kPairThreads, 1)
         run += all;
     }
     __syncthreads();
-    for (int lp = fresh.lo + static_cast<int>(threadIdx.x >> 5); lp < fresh.hi; lp += kPairThreads / 32) {
-        const int start = d.pairStart[lp], found = counts[lp];
-        int m = live + starts[lp];
-        for (int at = lane; at - lane < found; at += 32) {
+    for (int lp0 = fresh.lo + 4 * static_cast<int>(threadIdx.x >> 5); lp0 < fresh.hi; lp0 += 4 * (kPairThreads / 32)) {
+        const int lp = lp0 + part;
+        const bool on = lp < fresh.hi;
+        const int start = on ? d.pairStart[lp] : 0, found = on ? counts[lp] : 0;
+        int m = on ? live + starts[lp] : 0;
+        const int most = __reduce_max_sync(0xffffffffu, found);
+        for (int at = eighth; at - eighth < most; at += 8) {
             const int k = start + at;
             const bool ok = at < found && k < d.PP && d.pairValid[k];
-            const unsigned oks = __ballot_sync(0xffffffffu, ok);
-            const int to = m + __popc(oks & ((1u << lane) - 1u));
+            const unsigned oks = __ballot_sync(0xffffffffu, ok) >> (8 * part) & 0xffu;
+            const int to = m + __popc(oks & ((1u << eighth) - 1u));
             if (ok && to < d.MM) {
                 d.live.ab[to] = make_int2(n - 1 - lp, n - 1 - static_cast<int>(d.pairs[k] & 0xffffffffu));
                 d.live.count[to] = 0;
