@@ -2164,13 +2164,16 @@ size_t worldRows(int threads) { return sizeof(real) * static_cast<size_t>(thread
 // microseconds a step here and there:
 //   one world     211 bodies 286 / 456, 1261 (walls) 483 / 536, 2000 (pile) 578 / 676; where the parts do
 //                 not fit in shared memory, 1681 (walls) 637 / 551, 3000 (pile) 775 / 754
+//   with forces   600 bodies with ragdolls and springs 703 / 1680, a 1653-box pile with a chain 673 / 915
 //   many worlds   64 of 8-64 bodies 300 / 537, 256 of them 461 / 606, 512: 622 / 650, 1024: 945 / 751;
-//                 64 of 8-256 755 / 617
-//   with forces   600 bodies with ragdolls and springs 781 / 1680, a 1653-box pile with a chain 770 / 915
-// So worlds of up to 72 bodies a CTA, in up to three waves of CTAs, and a single world while it fits.
+//                 128 of 8-128 539 / 525, 64 of 8-256 540 / 528 (both 128 bodies a CTA)
+//   some worlds   32 of 64-512 353 / 540, 16 of 64-1024 394 / 527, 8 of 256-2048 415 / 533, 4 of 500-2048
+//                 387 / 509 (all 128 bodies a CTA); 9 of 1000-2048 (256 a CTA, too many for one) 685 / 586
+// So worlds of up to 72 bodies a CTA, or 128 where four CTAs and more share a world, in up to three waves of
+// CTAs, and a single world while it fits.
 bool worldsTake(int worlds, int bodies, double density, double forces) {
     const int team = worldTeam(worlds, bodies), per = divUp(bodies, team);
-    if (worlds * team > 3 * kSms || (worlds > 1 && per > 72))
+    if (worlds * team > 3 * kSms || (worlds > 1 && per > (team >= 4 ? 128 : 72)))
         return false;
     // Shared memory a CTA needs: its bodies, their stamp records (two a manifold), its manifolds and
     // their contacts (four a manifold and what packing leaves empty).
