@@ -1467,8 +1467,10 @@ int Engine::ensureIo(int count) {
     if (count <= ioCap)
         return AVBDG_OK;
     const int cap = std::max(count, 2 * ioCap);
-    if (ioHost)
+    if (ioHost) {
+        cudaStreamSynchronize(stream); // an unpack may still read it
         cudaFreeHost(ioHost);
+    }
     ioHost = nullptr;
     if (cudaMallocHost(&ioHost, sizeof(float) * 13 * static_cast<size_t>(cap)) != cudaSuccess)
         return fail(AVBDG_ERR_CAPACITY, "pinned staging allocation failed");

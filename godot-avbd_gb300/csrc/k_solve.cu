@@ -257,18 +257,12 @@ __global__ void finishKernel(Dev d, StepParams p, int idle) {
 // The counters to the host's memory. As a kernel behind the step's others it starts when they end; a copy,
 // like a memset between kernels, costs the work around it some microseconds of order (publish: 13 us a step;
 // each memset 5-8), which is why the kernels of a step clear each other's counts.
-__global__ void publishKernel(const int *ctr, int *to) {
-    pdlWait();
-    pdlTrigger();
-    __shared__ unsigned long long end;
+__global__ void publishKernel(int *ctr, int *to) {
     if (threadIdx.x == 0)
-        end = nowNs();
+        *reinterpret_cast<unsigned long long *>(ctr + C_CLOCK + 8) = nowNs(); // the step's end
     __syncthreads();
-    const int i = threadIdx.x;
-    if (i < C_CLOCK + 8)
-        to[i] = ctr[i];
-    else if (i < C_COUNT)
-        to[i] = reinterpret_cast<const int *>(&end)[i - C_CLOCK - 8];
+    if (threadIdx.x < C_COUNT)
+        to[threadIdx.x] = ctr[threadIdx.x];
 }
 
 // ---- update set and colouring (solver_solve.cpp:263-424) ----
@@ -615,7 +609,8 @@ void launchFinishBodies(const Dev &d, const StepParams &p, bool idle, cudaStream
 
 void launchPublish(const Dev &d, int *to, cudaStream_t s) {
     static_assert(C_COUNT <= kThreads, "one block");
-    ++launchCount(); launchK(publishKernel, 1, kThreads, 0, s, d.ctr, to);
+    ++launchCount(); // in plain stream order: it comes behind a graph as often as behind a kernel
+    publishKernel<<<1, kThreads, 0, s>>>(d.ctr, to);
 }
 
 void launchStamps(const Dev &d, const StepParams &p, bool mixedOnly, cudaStream_t s) {

@@ -206,3 +206,22 @@ def test_some_worlds(pkg, gpu, worlds, most):
     b.step(10)
     for w in range(0, worlds, 3):
         assert same([b.state(w)], [run(gpu, capi, kinds[w], 10)[9]])
+
+
+# The phase times of a step (one launch a world, or the separate launches): all parts counted, and together
+# no more than the host waited.
+@pytest.mark.parametrize("separate", ["0", "1"])
+def test_phase_times(pkg, gpu, monkeypatch, separate):
+    import time
+
+    monkeypatch.setenv("AVBDG_NO_WORLD", separate)
+    capi = pkg.capi
+    w = capi.World(gpu, gpu.default_params(), max_bodies=301)
+    w.add_bodies(heap(capi, 300, 5))
+    for _ in range(12):
+        begin = time.perf_counter()
+        w.step()
+        wall = 1000 * (time.perf_counter() - begin)
+        st = w.stats()
+        parts = [st.broad_ms, st.graph_ms, st.solve_ms] + ([st.finish_ms] if separate == "1" else [])
+        assert min(parts) > 0 and abs(sum(parts) - st.total_ms) < 1e-9 and 0.05 < st.total_ms < wall
