@@ -30,6 +30,17 @@ __device__ __forceinline__ void clusterSync(int size) {
     }
 }
 
+// Shared-memory addresses, of this CTA or (mapped) of another of the cluster.
+__device__ __forceinline__ unsigned sharedAddress(const void *p) { return static_cast<unsigned>(__cvta_generic_to_shared(p)); }
+__device__ __forceinline__ unsigned mapShared(unsigned a, int rank) {
+    unsigned r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void storeClusterInt(unsigned a, int v) {
+    asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+
 // Cluster and (programmatic) stream attributes of a launch.
 struct TeamLaunch {
     cudaLaunchConfig_t cfg{};

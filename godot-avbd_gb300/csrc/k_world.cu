@@ -95,13 +95,6 @@ struct World {
     int rec0, con0;                // this CTA's address of the pose records and step constants
 };
 
-// Shared-memory addresses, of this CTA or (mapped) of another of the cluster.
-__device__ __forceinline__ unsigned sharedAddress(const void *p) { return static_cast<unsigned>(__cvta_generic_to_shared(p)); }
-__device__ __forceinline__ unsigned mapShared(unsigned a, int rank) {
-    unsigned r;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
-    return r;
-}
 __device__ __forceinline__ real4 loadCluster(unsigned a) {
     real4 v;
 #ifdef AVBDG_FP64
@@ -119,9 +112,6 @@ __device__ __forceinline__ void storeCluster(unsigned a, real4 v) {
 #else
     asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
 #endif
-}
-__device__ __forceinline__ void storeClusterInt(unsigned a, int v) {
-    asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
 }
 __device__ __forceinline__ void maxClusterInt(unsigned a, int v) {
     asm volatile("red.shared::cluster.max.s32 [%0], %1;" ::"r"(a), "r"(v) : "memory");

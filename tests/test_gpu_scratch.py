@@ -121,3 +121,16 @@ def test_pick_tiles(pkg, gpu, oracle, n):
     assert np.array_equal(la, np.concatenate([p[1] for p in part]), equal_nan=True)
     ga[6], la[6] = gb[6], lb[6]  # which of its distances of NaN a ray takes is not the oracle's
     assert np.array_equal(ga, gb) and np.array_equal(la, lb, equal_nan=True) and (ga >= 0).sum() > rays // 20
+
+
+# The scan behind a collect, by one block, by a cluster of two to sixteen CTAs and by three launches.
+@pytest.mark.parametrize("n", [4095, 4096, 4097, 20_000, 140_000, 540_000])
+def test_collect_scans(pkg, gpu, n):
+    capi, rng = pkg.capi, np.random.default_rng(n)
+    pos = rng.uniform(-50, 50, (n, 3))
+    w = capi.World(gpu, gpu.default_params(), max_bodies=n)
+    w.add_bodies(capi.make_body_descs([[0.1, 0.1, 0.1]] * n, [1.0] * n, 0.5, pos))
+    pos, half = pos.astype(np.float32), np.float32(0.05)
+    lo, hi = np.float32([-30, -30.5, -20]), np.float32([25, 35, 41])
+    inside = ((pos - half <= hi) & (lo <= pos + half)).all(axis=1)
+    assert np.array_equal(w.collect_aabb(lo, hi), np.nonzero(inside)[0][::-1])  # list order: the last first
