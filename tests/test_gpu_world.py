@@ -194,18 +194,20 @@ def test_colouring(pkg, gpu, monkeypatch, n, params):
     assert same(here, run_forces(gpu, capi, world, params, steps=8))
 
 
-# Some worlds of very different sizes, up to 128 bodies a CTA, with and without forces: each equals itself alone.
+# Some worlds of very different sizes, up to 128 bodies a CTA, without forces and with: each equals itself alone.
+@pytest.mark.parametrize("forces", [False, True])
 @pytest.mark.parametrize("worlds,most", [(4, 1700), (16, 900), (30, 480)])
-def test_some_worlds(pkg, gpu, worlds, most):
+def test_some_worlds(pkg, gpu, worlds, most, forces):
     capi = pkg.capi
-    kinds = [heap(capi, max(2, int(most * k / worlds) - k % 3), k) for k in range(worlds, 0, -1)]
-    b = capi.Batch(gpu.lib, max_worlds=worlds, max_bodies=4 * sum(len(d) for d in kinds))
-    for d in kinds:
-        b._api.check(b.fn["batch_add_world"](b.handle, len(d), d, 0, None, capi.C.byref(capi.C.c_int())))
+    kinds = [tangle(capi, max(2, int(most * k / worlds) - k % 3), k) for k in range(worlds, 0, -1)]
+    kinds = [(d, f[:25] if forces and k % 3 else []) for k, (d, f) in enumerate(kinds)]
+    b = capi.Batch(gpu.lib, max_worlds=worlds, max_bodies=4 * sum(len(d) for d, _ in kinds), max_forces=25 * worlds)
+    for d, f in kinds:
+        b._api.check(b.fn["batch_add_world"](b.handle, len(d), d, len(f), capi.make_force_descs(f), capi.C.byref(capi.C.c_int())))
         b.sizes.append(len(d))
     b.step(10)
-    for w in range(0, worlds, 3):
-        assert same([b.state(w)], [run(gpu, capi, kinds[w], 10)[9]])
+    for w in range(0, worlds, 3 if worlds > 4 else 1):
+        assert same([b.state(w)], run_forces(gpu, capi, kinds[w], {}, steps=10)[9:])
 
 
 # The phase times of a step (one launch a world, or the separate launches): all parts counted, and together
