@@ -52,7 +52,6 @@ enum Counter {
     C_WORLDS,         // worlds
     C_ERRORS,         // capacity / timeout bits (kErr*)
     C_ONE,            // constant 1 (scan length helper)
-    C_SOLVEFAIL,      // overflow bodies whose plain LDLT failed this round (solveFail)
     C_PAIRSPILL,      // bodies with more broad-phase partners than the stash holds (pairSpill)
     C_QSOLVE,         // round-loop queue: solve tiles a round (all worlds)
     C_QDUAL,          // round-loop queue: dual tiles a round (all worlds)
@@ -158,7 +157,7 @@ struct Dev {
     int2 *stampSlot;        // per live manifold: the adjacency entries of its side-A and side-B stamps
     uint8_t *mSpec, *mDone; // brake: candidate flag per manifold, done flag per candidate
     int *specList;
-    int *solveFail;         // overflow bodies left to the pivoted fallback this round
+    int *solveFail;         // a word per body: scratch of the cluster launches
     int *pairStash;         // broad phase: first kPairStash partners' list positions per body list position
     int *pairSpill;         // broad phase: bodies whose partners overflow the stash (walked again)
     int2 *specPred;         // brake: candidate index of the preceding candidate on each movable body (-1 = none)
