@@ -21,16 +21,20 @@ __device__ __forceinline__ int clusterSize() {
 
 // Cluster barrier: writes before it, to global memory and to any CTA's shared memory, are visible to the
 // cluster's threads after it.
+__device__ __forceinline__ void clusterArrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void clusterWait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
 __device__ __forceinline__ void clusterSync(int size) {
     if (size == 1) {
         __syncthreads();
     } else {
-        asm volatile("barrier.cluster.arrive.release;" ::: "memory");
-        asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+        clusterArrive();
+        clusterWait();
     }
 }
 
-// Shared-memory addresses, of this CTA or (mapped) of another of the cluster.
+// Shared-memory addresses, of this CTA or (mapped) of another of the cluster. Another CTA's memory may be
+// touched once that CTA is known to run (a cluster barrier after the kernel's start) and until it may end (a
+// cluster barrier before the kernel's end, or after the last access).
 __device__ __forceinline__ unsigned sharedAddress(const void *p) { return static_cast<unsigned>(__cvta_generic_to_shared(p)); }
 __device__ __forceinline__ unsigned mapShared(unsigned a, int rank) {
     unsigned r;

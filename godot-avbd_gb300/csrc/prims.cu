@@ -149,6 +149,7 @@ __global__ void __launch_bounds__(kSmallThreads) scanClusterKernel(const int *in
     pdlTrigger();
     __shared__ int warpSums[kSmallThreads / 32], totals[2][kMaxTeam];
     const int n = loadCount(d_n, capacity), rank = clusterRank(), size = clusterSize(), lanes = size * kSmallThreads;
+    clusterArrive(); // a CTA's shared memory is another's to write once it runs: waited for before the first turn's sums
     int run = 0, turn = 0;
     for (int first = 0, per; first < n; first += lanes * per, turn ^= 1) {
         per = min(kClusterItems, (n - first + lanes - 1) / lanes);
@@ -161,6 +162,8 @@ __global__ void __launch_bounds__(kSmallThreads) scanClusterKernel(const int *in
         }
         int total;
         int prefix = run + blockExclusiveScan<kSmallThreads>(s, warpSums, total);
+        if (first == 0)
+            clusterWait();
         if (static_cast<int>(threadIdx.x) < size)
             storeClusterInt(mapShared(sharedAddress(&totals[turn][rank]), threadIdx.x), total);
         clusterSync(size); // (a turn's sums are read before anyone writes those of the turn after the next)
@@ -175,6 +178,8 @@ __global__ void __launch_bounds__(kSmallThreads) scanClusterKernel(const int *in
             prefix += v[k];
         }
     }
+    if (n <= 0)
+        clusterWait();
     if (rank == 0 && threadIdx.x == 0 && d_total)
         *d_total = run;
 }

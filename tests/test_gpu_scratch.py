@@ -134,3 +134,30 @@ def test_collect_scans(pkg, gpu, n):
     lo, hi = np.float32([-30, -30.5, -20]), np.float32([25, 35, 41])
     inside = ((pos - half <= hi) & (lo <= pos + half)).all(axis=1)
     assert np.array_equal(w.collect_aabb(lo, hi), np.nonzero(inside)[0][::-1])  # list order: the last first
+
+
+# The cluster's scan while other work fills the device, so that its CTAs start apart: each of a world's
+# collects counts the same bodies, on four streams at once.
+def test_scans_on_a_busy_device(pkg, gpu):
+    capi, bad = pkg.capi, []
+
+    def work(n):
+        rng = np.random.default_rng(n)
+        pos = rng.uniform(-50, 50, (n, 3))
+        w = capi.World(gpu, gpu.default_params(), max_bodies=n)
+        w.add_bodies(capi.make_body_descs([[0.1, 0.1, 0.1]] * n, [1.0] * n, 0.5, pos))
+        at, half = pos.astype(np.float32), np.float32(0.05)
+        for k in range(200):
+            lo = np.float32([-40 + k % 7, -30.5, -20])
+            hi = lo + np.float32([50, 60, 40 + k % 11])
+            inside = ((at - half <= hi) & (lo <= at + half)).all(axis=1)
+            if not np.array_equal(w.collect_aabb(lo, hi), np.nonzero(inside)[0][::-1]):
+                bad.append((n, k))
+        w.step(20)
+
+    threads = [threading.Thread(target=work, args=(n,)) for n in (4200, 9000, 33_000, 100_000)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
