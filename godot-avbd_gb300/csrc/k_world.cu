@@ -712,7 +712,7 @@ __device__ __forceinline__ int passRows() { return 32 * contactWarps(); }
 
 template <bool ARM>
 __device__ __forceinline__ void colourPhase(const Dev &d, const StepParams &p, const World &w, unsigned char *smem, int colours,
-                                            int armsFromDual, real *carry) {
+                                            int armsFromDual, real (*carries)[32]) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5, group = passRows();
     real *rows = arrayAt<real>(smem, 0);
     const int *termFirst = arrayAt<int>(smem, w.termFirst);
@@ -726,6 +726,9 @@ __device__ __forceinline__ void colourPhase(const Dev &d, const StepParams &p, c
         const int first = k0 < k1 ? termFirst[k0] : 0, last = k0 < k1 ? termFirst[k1] : 0;
         for (int from = first, pass = 0; k0 < k1 && (pass == 0 || from < last); from += group, pass++) {
             const int to = min(from + group, last);
+            // A body that goes on hands its sums to the next pass. In one pass the body that came over reads the last
+            // one's while another warp may write the next one's: two in turn.
+            real *carried = carries[(pass + 1) & 1], *carry = carries[pass & 1];
             // Terms: warps take up to 32 of a kind.
             const uint16_t *kinds = arrayAt<uint16_t>(smem, w.termKinds) + (w.groupAt[c] + pass) * (kTermKinds + 1);
             for (int task = warp, kind = 0, before = 0; kind < kTermKinds; kind++) {
@@ -766,7 +769,7 @@ __device__ __forceinline__ void colourPhase(const Dev &d, const StepParams &p, c
                 if (!done && !(t0 < to && t1 > from))
                     continue;
                 real *sums = arrayAt<real>(smem, w.colourBlocks) + k * kBlkReals;
-                real v = lane < 30 ? sums[lane] : 0.0f, acc = t0 < from ? carry[lane] : 0.0f;
+                real v = lane < 30 ? sums[lane] : 0.0f, acc = t0 < from ? carried[lane] : 0.0f;
                 const real *r = rows + (max(t0, from) - from) * kRowReals, *end = rows + (min(t1, to) - from) * kRowReals;
 #pragma unroll 4
                 for (; r < end; r += kRowReals) {
@@ -1849,7 +1852,7 @@ __global__ void __launch_bounds__(kMaxWorldThreads, 1)
     stampPhase(d);
     extern __shared__ __align__(32) unsigned char smem[];
     __shared__ int shared[4], deepest[2];
-    __shared__ real carry[32];
+    __shared__ real carry[2][32];
     __shared__ SetupShared sh;
     // The world's description is uniform and wide: it is kept in shared memory, and a phase reads what
     // it needs.

@@ -227,3 +227,51 @@ def test_phase_times(pkg, gpu, monkeypatch, separate):
         st = w.stats()
         parts = [st.broad_ms, st.graph_ms, st.solve_ms] + ([st.finish_ms] if separate == "1" else [])
         assert min(parts) > 0 and abs(sum(parts) - st.total_ms) < 1e-9 and 0.05 < st.total_ms < wall
+
+
+def press(capi, layers, anchors):
+    """Plates held by ball joints to the world (`anchors` of them each), `layers` of 34 boxes between them. The plates
+    come last, so all take the first colour."""
+    rng = np.random.default_rng(7)
+    i = np.arange(34)
+    size, pos = [], []
+    for k in range(layers):
+        pos.append(np.stack([0.9 * (i % 7) - 2.7, 0.9 * (i // 7) - 1.8, 0.5 + 0.99 * k + 0 * i], 1) + [0.01, 0.01, 0] * rng.uniform(-1, 1, (34, 3)))
+        size += [[0.6, 0.6, 0.6]] * 34
+    plates = [[0, 0, 0.99 * k] for k in range(layers + 1)]
+    size += [[8, 6, 0.4]] * (layers + 1)
+    d = capi.make_body_descs(size, [1.0] * len(size), 0.5, np.concatenate(pos + [plates]))
+    forces = []
+    for k, n in enumerate(anchors):
+        for _ in range(n):
+            r = rng.uniform([-4, -3, -0.2], [4, 3, 0.2])
+            forces.append((-1, 34 * layers + k, tuple(r + plates[k]), tuple(r), 2000.0, 0.0, float("inf")))
+    return d, forces
+
+
+# A CTA (65 to 72 bodies: 288 terms a pass) whose first colour takes three passes and more, with a body that comes
+# over from the pass before beside one that goes on to the next, both cut inside a manifold's contacts.
+def test_colour_of_many_passes(pkg, gpu, oracle):
+    capi = pkg.capi
+    d, forces = press(capi, 2, (17, 10, 10))
+    worlds = 78  # more than half the SMs: a CTA a world
+    b = capi.Batch(gpu.lib, max_worlds=worlds, max_bodies=worlds * len(d), max_forces=worlds * len(forces))
+    for _ in range(worlds):
+        b._api.check(b.fn["batch_add_world"](b.handle, len(d), d, len(forces), capi.make_force_descs(forces), capi.C.byref(capi.C.c_int())))
+        b.sizes.append(len(d))
+    w = capi.World(oracle, oracle.default_params())
+    w.add_bodies(d)
+    for f in forces:
+        w.add_force(f)
+    cut = 0
+    for _ in range(24):
+        b.step()
+        w.step()
+        for k in (0, 40, 77):
+            assert same([b.state(k)], [w.state()])
+        m, (colour, ids) = w.manifolds(), w.colours()
+        assert (colour[ids >= 68] == 0).all()
+        terms = [3 * n + m["count"][(m["body_a"] == 68 + k) | (m["body_b"] == 68 + k)].sum() for k, n in enumerate((17, 10, 10))]
+        ends = np.cumsum(terms)
+        cut += ends[0] < 288 < ends[1] < 576 < ends[2]
+    assert cut > 12  # steps that cross both borders
