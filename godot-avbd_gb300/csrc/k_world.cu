@@ -1911,8 +1911,11 @@ __global__ void __launch_bounds__(kMaxWorldThreads, 1)
             continue;
         for (int step = 0;; step++) {
             const bool finished = step == r.substeps; // the brake runs once more after the last substep
-            if (step > 0 && !finished)
+            if (step > 0 && !finished) {
                 rebasePhase(d, p, w, smem);
+                if (!r.brake) // (whose barriers keep the poses that the rebase reads)
+                    clusterSync(size);
+            }
             if (r.brake)
                 brakePhase(d, w, smem, r.substeps > 1 && !finished ? r.dt * static_cast<real>(r.substeps - step) : p.collisionDt);
             if (finished)

@@ -275,3 +275,16 @@ def test_colour_of_many_passes(pkg, gpu, oracle):
         ends = np.cumsum(terms)
         cut += ends[0] < 288 < ends[1] < 576 < ends[2]
     assert cut > 12  # steps that cross both borders
+
+
+# Substeps without the brake, whose barriers otherwise part a substep's rebase from the next one's warm start: one
+# CTA and several, without forces and with.
+@pytest.mark.parametrize("interleaved", [(2, 3), (4, 2)])
+@pytest.mark.parametrize("n", [20, 45, 300])
+def test_substeps_without_brake(pkg, gpu, oracle, n, interleaved):
+    capi, params = pkg.capi, {"speculative_margin": 0.0}
+    d = heap(capi, n, n)
+    assert same(run(gpu, capi, d, 20, params, interleaved), run(oracle, capi, d, 20, params, interleaved))
+    world = tangle(capi, n, n, ragdolls=False)
+    world = world[0], world[1][:30]
+    assert same(run_forces(gpu, capi, world, params, interleaved=interleaved), run_forces(oracle, capi, world, params, interleaved=interleaved))
