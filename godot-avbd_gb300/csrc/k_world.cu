@@ -2118,7 +2118,12 @@ WorldKernel wideKernelFor(bool colours, bool arm) {
                    : (arm ? worldWideKernel<false, true> : worldWideKernel<false, false>);
 }
 
-constexpr int kSmemMost = 222 * 1024; // dynamic shared memory a CTA may have beside the static part
+// Dynamic shared memory a CTA may have beside the static part, of 227 KB together.
+#ifdef AVBDG_FP64
+constexpr int kSmemMost = 221 * 1024;
+#else
+constexpr int kSmemMost = 222 * 1024;
+#endif
 
 int g_maxTeam = 0;
 
