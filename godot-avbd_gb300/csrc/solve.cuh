@@ -891,8 +891,10 @@ __device__ __forceinline__ void stampsAt(const Dev &d, const StepParams &p, int 
 // ARM: the arm cache is on (compiled out otherwise, so the common path keeps its code).
 // One manifold's dual pass (and, with STAMPS, its next-round stamps): the body of dualKernel's loop,
 // also run by the tile queue of the round loop.
-// RO: poses are read-only for the whole launch (read-only cache path); false inside the round-loop
-// tile queue, which writes them in the same launch.
+// RO: poses and gaps (C0) are read-only for the whole launch (read-only cache path); false inside the
+// round-loop tile queue, which writes poses in the same launch, and worldWideKernel, which writes both (its
+// rebase between substeps). What else goes through the read-only path no launch that runs this writes: a
+// manifold's pair, basis and count and its contacts' arms in body frames are the narrow phase's.
 template <bool STAMPS, bool ARM, bool RO = true>
 __device__ __forceinline__ void dualAt(const Dev &d, const StepParams &p, real decay, int m) {
     const ManifoldBuf L = d.live;
@@ -908,6 +910,7 @@ __device__ __forceinline__ void dualAt(const Dev &d, const StepParams &p, real d
     const f3 r0 = xyz(b04), r1 = xyz(__ldg(&L.b1[m])), r2 = xyz(__ldg(&L.b2[m]));
     const real mu = b04.w;
     const int n = __ldg(&L.count[m]);
+    const auto gap = [&](int ci) { return xyz(RO ? __ldg(&L.C0[ci]) : L.C0[ci]); };
     // Drift-gated arm reuse (manifold.cpp:600-608): under the rotation threshold the cached
     // world arms stand in for the current ones.
     bool driftUsable = false;
@@ -946,7 +949,7 @@ __device__ __forceinline__ void dualAt(const Dev &d, const StepParams &p, real d
             }
         }
         const f3 bracket = sub(add(sub(A.dLin, B.dLin), cross(A.dAng, rAw)), cross(B.dAng, rBw));
-        const f3 C = contactError(p, xyz(__ldg(&L.C0[ci])), bracket, r0, r1, r2);
+        const f3 C = contactError(p, gap(ci), bracket, r0, r1, r2);
         f3 k = xyz(L.k[ci]);
         if (decay < 1.0f)
             k = lclampv(scale(k, decay), PENALTY_MIN, PENALTY_MAX);
@@ -974,7 +977,7 @@ __device__ __forceinline__ void dualAt(const Dev &d, const StepParams &p, real d
                     rAs = mul(A.rot, xyz(rA4));
                     rBs = mul(B.rot, xyz(L.rB[ci]));
                     const f3 bracketF = sub(add(sub(A.dLin, B.dLin), cross(A.dAng, rAs)), cross(B.dAng, rBs));
-                    Cs = contactError(p, xyz(L.C0[ci]), bracketF, r0, r1, r2);
+                    Cs = contactError(p, gap(ci), bracketF, r0, r1, r2);
                 }
                 L.armA[ci] = f4(rAs, 0.0f);
                 L.armB[ci] = f4(rBs, 0.0f);

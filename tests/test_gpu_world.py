@@ -288,3 +288,22 @@ def test_substeps_without_brake(pkg, gpu, oracle, n, interleaved):
     world = tangle(capi, n, n, ragdolls=False)
     world = world[0], world[1][:30]
     assert same(run_forces(gpu, capi, world, params, interleaved=interleaved), run_forces(oracle, capi, world, params, interleaved=interleaved))
+
+
+# A world that does not fit in shared memory, with substeps (each begins from the gaps that the rebase of the one before
+# wrote in the same launch): arms kept or not, sleepers, and with forces, where jointed bodies find no colour free and the
+# oracle has other last bits: the same as the separate launches.
+@pytest.mark.parametrize("forces", [False, True])
+@pytest.mark.parametrize("params", [{}, {"jacobian_rebuild_distance": 0.05},
+                                    {"sleep_frames": 2, "sleep_linear_threshold": 5.0, "sleep_angular_threshold": 5.0}])
+def test_dense_world_with_substeps(pkg, gpu, oracle, monkeypatch, params, forces):
+    capi = pkg.capi
+    dense = heap(capi, 150, 3, 0.25)
+    for i in range(1, 151):
+        dense[i].sleep_mode = i % 3 if "sleep_frames" in params else 0
+    world = dense, tangle(capi, 150, 3, ragdolls=False)[1][:12] if forces else []
+    here = run_forces(gpu, capi, world, params, steps=6, interleaved=(3, 2))
+    monkeypatch.setenv("AVBDG_NO_WORLD", "1")
+    assert same(here, run_forces(gpu, capi, world, params, steps=6, interleaved=(3, 2)))
+    if not forces:
+        assert same(here, run_forces(oracle, capi, world, params, steps=6, interleaved=(3, 2)))
