@@ -64,8 +64,8 @@ struct TeamLaunch {
     }
 };
 
-// Allows `kernel` clusters of up to kMaxTeam CTAs with `smem` dynamic shared bytes; the largest cluster
-// (a power of two) the device can hold.
+// Allows `kernel` clusters of up to kMaxTeam CTAs with `smem` dynamic shared bytes on the current device; the
+// largest cluster (a power of two) the device can hold.
 inline int allowTeam(const void *kernel, int threads, size_t smem) {
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);

@@ -774,7 +774,6 @@ __global__ void __launch_bounds__(kPairThreads, 1)
     }
 }
 
-int g_pairTeam = 0;
 constexpr int kPairSmem = 220 * 1024; // of a CTA; the world's boxes are in it
 
 } // namespace
@@ -837,9 +836,8 @@ void launchFilterAcquire(const Dev &d, cudaStream_t s) {
 }
 
 static int pairTeamMax() {
-    if (g_pairTeam == 0)
-        g_pairTeam = allowTeam(reinterpret_cast<const void *>(worldPairsKernel), kPairThreads, kPairSmem);
-    return g_pairTeam;
+    static PerDevice teams;
+    return teams.get(currentDevice(), [] { return allowTeam(reinterpret_cast<const void *>(worldPairsKernel), kPairThreads, kPairSmem); });
 }
 
 // The all-pairs test grows with the square of the bodies, the tree does not. Measured, microseconds a
@@ -851,8 +849,9 @@ int worldPairsMost() {
 }
 
 void launchWorldPairs(const Dev &d, const StepParams &p, int bodies, cudaStream_t s) {
+    const int largest = pairTeamMax();
     int team = 1;
-    while (team < pairTeamMax() && team * 24 < bodies)
+    while (team < largest && team * 24 < bodies)
         team *= 2;
     const TeamLaunch l(team, 1, kPairThreads, sizeof(Box) * static_cast<size_t>(bodies), s);
     ++launchCount();

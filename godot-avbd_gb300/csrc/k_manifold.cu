@@ -702,22 +702,21 @@ bool narrowBlockFits(int block) {
     return blockFits(manifoldInitKernel<false>, block) && blockFits(manifoldInitKernel<true>, block);
 }
 
-static int g_contactTeam = 0;
-
 static int contactTeamMax() {
-    if (g_contactTeam == 0) {
+    static PerDevice teams;
+    return teams.get(currentDevice(), [] {
         const int a = allowTeam(reinterpret_cast<const void *>(worldContactsKernel<false>), kContactThreads, 0);
         const int b = allowTeam(reinterpret_cast<const void *>(worldContactsKernel<true>), kContactThreads, 0);
-        g_contactTeam = a < b ? a : b;
-    }
-    return g_contactTeam;
+        return a < b ? a : b;
+    });
 }
 
 void prepareWorldContacts() { contactTeamMax(); }
 
 void launchWorldContacts(const Dev &d, const StepParams &p, bool round, bool select, int bodies, cudaStream_t s) {
+    const int largest = contactTeamMax();
     int team = 1;
-    while (team < contactTeamMax() && team * 16 < bodies)
+    while (team < largest && team * 16 < bodies)
         team *= 2;
     const TeamLaunch l(team, 1, kContactThreads, 0, s);
     ++launchCount();

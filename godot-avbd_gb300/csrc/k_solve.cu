@@ -519,7 +519,6 @@ void launchContactOnly(const Dev &d, cudaStream_t s) {
     ++launchCount(); launchK(contactOnlyMarkKernel, grid(d.FF), kThreads, 0, s, d);
 }
 
-constexpr int kSms = 152;
 static int g_colourBlocks = 0;
 
 int colourGridBlocks() {
@@ -579,7 +578,7 @@ void launchColour(const Dev &d, bool needGreedy, bool everyWorld, int largest, c
     if (!needGreedy)
         return;
     if (largest > 0) {
-        const int blocks = d.WW < 4 * kSms ? d.WW : 4 * kSms;
+        const int most = 4 * smCount(), blocks = d.WW < most ? d.WW : most;
         ++launchCount();
         launchK(colourWorldKernel, blocks, kColourWorldThreads, kColourBodyBytes * static_cast<size_t>(largest), s, d,
                 everyWorld ? 1 : 0, largest);

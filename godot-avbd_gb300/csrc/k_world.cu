@@ -2125,31 +2125,28 @@ constexpr int kSmemMost = 221 * 1024;
 constexpr int kSmemMost = 222 * 1024;
 #endif
 
-int g_maxTeam = 0;
-
 } // namespace
 
 int worldTeamMax() {
-    if (g_maxTeam == 0) {
+    static PerDevice teams;
+    return teams.get(currentDevice(), [] {
         int team = kMaxTeam;
         for (int c = 0; c < 4; c++) {
             team = std::min(team, allowTeam(reinterpret_cast<const void *>(worldKernelFor(c & 1, c & 2)), kMaxWorldThreads, kSmemMost));
             team = std::min(team, allowTeam(reinterpret_cast<const void *>(wideKernelFor(c & 1, c & 2)), kWideThreads, kSmemMost));
         }
-        g_maxTeam = team;
-    }
-    return g_maxTeam;
+        return team;
+    });
 }
 
 namespace {
 
-constexpr int kSms = 152;
-
 // CTAs a world: enough that a CTA has about 24 bodies (their contacts then take one pass of its
 // contact warps), as far as the GPU's SMs go round the worlds (a CTA fills one).
 int worldTeam(int worlds, int bodies) {
+    const int largest = worldTeamMax(), sms = smCount();
     int team = 1;
-    while (team < worldTeamMax() && team * 24 < bodies && 2 * team * worlds <= kSms)
+    while (team < largest && team * 24 < bodies && 2 * team * worlds <= sms)
         team *= 2;
     return team;
 }
@@ -2174,7 +2171,7 @@ size_t worldRows(int threads) { return sizeof(real) * static_cast<size_t>(thread
 // CTAs, and a single world while it fits.
 bool worldsTake(int worlds, int bodies, double density, double forces) {
     const int team = worldTeam(worlds, bodies), per = divUp(bodies, team);
-    if (worlds * team > 3 * kSms || (worlds > 1 && per > (team >= 4 ? 128 : 72)))
+    if (worlds * team > 3 * smCount() || (worlds > 1 && per > (team >= 4 ? 128 : 72)))
         return false;
     // Shared memory a CTA needs: its bodies, their stamp records (two a manifold), its manifolds and
     // their contacts (four a manifold and what packing leaves empty).

@@ -554,19 +554,27 @@ size_t radixScratchBytes(int capacity) {
 
 size_t uniqueScratchBytes(int count) { return static_cast<size_t>(divUp(count > 0 ? count : 1, kRadixTile)) * sizeof(int); }
 
-static int g_scanTeam = 0;
+int smCount() {
+    static PerDevice counts;
+    const int device = currentDevice();
+    return counts.get(device, [device] {
+        int sms = 0;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+        return sms > 0 ? sms : 1;
+    });
+}
 
 static int scanTeam() {
-    if (g_scanTeam == 0)
-        g_scanTeam = allowTeam(reinterpret_cast<const void *>(scanClusterKernel), kSmallThreads, 0);
-    return g_scanTeam;
+    static PerDevice teams;
+    return teams.get(currentDevice(), [] { return allowTeam(reinterpret_cast<const void *>(scanClusterKernel), kSmallThreads, 0); });
 }
 
 void scanExclusive(const int *in, int *out, int capacity, const int *d_n, int *d_total, void *scratch,
                    cudaStream_t stream) {
-    if (capacity > kBlockScanCap && capacity <= kClusterScanCap && scanTeam() > 1) {
+    const int largest = capacity > kBlockScanCap && capacity <= kClusterScanCap ? scanTeam() : 1;
+    if (largest > 1) {
         int team = 2;
-        while (team < scanTeam() && team * 2 * kSmallThreads < capacity)
+        while (team < largest && team * 2 * kSmallThreads < capacity)
             team *= 2;
         const TeamLaunch l(team, 1, kSmallThreads, 0, stream);
         ++launchCount();
@@ -643,12 +651,11 @@ static void segmentedSort(T *data, const int *start, int segCapacity, const int 
     }
 }
 
-static bool g_smemConfigured = false;
-
-static void configureSmem();
-
 void preparePrimitives() {
-    configureSmem();
+    cudaFuncSetAttribute(segMidKernel<uint32_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         static_cast<int>(kMidSegCap * sizeof(uint32_t)));
+    cudaFuncSetAttribute(segMidKernel<uint64_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         static_cast<int>(kMidSegCap * sizeof(uint64_t)));
     scanTeam();
 }
 
@@ -681,25 +688,13 @@ int residentGrid(const void *kernel, int block, size_t smem, int want) {
     return want < 1 ? 1 : (want < blocks ? want : blocks);
 }
 
-static void configureSmem() {
-    if (g_smemConfigured)
-        return;
-    cudaFuncSetAttribute(segMidKernel<uint32_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         static_cast<int>(kMidSegCap * sizeof(uint32_t)));
-    cudaFuncSetAttribute(segMidKernel<uint64_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         static_cast<int>(kMidSegCap * sizeof(uint64_t)));
-    g_smemConfigured = true;
-}
-
 void segmentedSortU32(uint32_t *data, uint32_t *tmp, const int *start, int segCapacity, const int *d_segments,
                       int *longList, int *longCount, cudaStream_t stream) {
-    configureSmem();
     segmentedSort<uint32_t>(data, start, segCapacity, d_segments, longList, longCount, tmp, stream);
 }
 
 void segmentedSortU64(uint64_t *data, uint64_t *tmp, const int *start, int segCapacity, const int *d_segments,
                       int *longList, int *longCount, cudaStream_t stream) {
-    configureSmem();
     segmentedSort<uint64_t>(data, start, segCapacity, d_segments, longList, longCount, tmp, stream);
 }
 

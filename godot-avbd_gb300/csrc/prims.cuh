@@ -10,6 +10,8 @@
 #include <utility>
 #include <cuda_runtime.h>
 
+#include "perdevice.hpp"
+
 namespace avbdg {
 
 // Programmatic dependent launch. The step is a chain of dependent kernels, most of them a few
@@ -52,6 +54,13 @@ inline void launchK(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem
     cfg.numAttrs = 1;
     cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
+
+inline int currentDevice() {
+    int device = 0;
+    cudaGetDevice(&device);
+    return device;
+}
+int smCount(); // of the current device
 
 // Scratch sizes the primitives need for `capacity` elements.
 size_t scanScratchBytes(int capacity);

@@ -86,3 +86,17 @@ def test_cpp_facade_compiles(tmp_path):
     subprocess.run([cxx, "-std=c++17", "-Wall", "-Wextra", "-Werror", "-ffp-contract=off",
                     "-I" + os.path.join(ROOT, "include"), "-c", os.path.join(ROOT, "tests", "cpp", "facade_scenes.cpp"),
                     "-o", str(tmp_path / "facade.o")], check=True)
+
+
+def test_values_kept_by_device(tmp_path):
+    """What is found once a device (the largest cluster, the SMs) is found for each device."""
+    import shutil
+    import subprocess
+
+    cxx = shutil.which("g++")
+    if cxx is None:
+        pytest.skip("no C++ compiler")
+    exe = str(tmp_path / "perdevice")
+    subprocess.run([cxx, "-std=c++17", "-Wall", "-Wextra", "-Werror", "-pthread", "-I" + os.path.join(ROOT, "godot-avbd_gb300", "csrc"),
+                    os.path.join(ROOT, "tests", "cpp", "perdevice.cpp"), "-o", exe], check=True)
+    subprocess.run([exe], check=True)
