@@ -115,20 +115,49 @@ int staticScratchAddress(void **out) {
 // ---- Kept scratch -----------------------------------------------------------------------------
 //
 // A cudaMalloc and a cudaFree of a million keys' scratch take about 155 us, more than the kernels do.
-// So a call leaves its block for the next one: at most one a device, of at most kKeptBytes. A
+// So a call leaves its block for the next one: at most one a context, of at most kKeptBytes. A
 // call takes the block out (a second thread finds none and allocates), and it has waited for its stream
 // before it puts it back, so no stream ever shares it. It belongs to the context it was allocated in, which
-// is known by its id: after a device reset it is forgotten. It is given back when a world, batch or server
-// is destroyed and when one of them cannot allocate.
+// is known by its id: no other context takes it, and after a device reset nobody does (its place, of
+// kMostKept, stays taken). It is given back when a world, batch or server of its context is destroyed and when
+// one of them cannot allocate.
 constexpr size_t kKeptBytes = size_t(64) << 20;
+constexpr int kMostKept = 64;
 
 struct KeptScratch {
     void *base;
     size_t bytes;
     unsigned long long context;
 };
-static KeptScratch g_kept[kMaxDevices] = {};
+static KeptScratch g_kept[kMostKept] = {};
 static std::mutex g_keptMutex;
+
+// The context's block, taken out; none: base is null.
+KeptScratch takeKept(unsigned long long context) {
+    KeptScratch out{};
+    std::lock_guard<std::mutex> lock(g_keptMutex);
+    for (KeptScratch &k : g_kept)
+        if (k.base && k.context == context) {
+            std::swap(out, k);
+            break;
+        }
+    return out;
+}
+
+// Keeps a context's block; false where it has one or all places are taken.
+bool putKept(const KeptScratch &block) {
+    std::lock_guard<std::mutex> lock(g_keptMutex);
+    KeptScratch *place = nullptr;
+    for (KeptScratch &k : g_kept) {
+        if (k.base && k.context == block.context)
+            return false;
+        if (!k.base && !place)
+            place = &k;
+    }
+    if (place)
+        *place = block;
+    return place != nullptr;
+}
 
 // The id of the current context, unique in the process; 0 where there is none.
 unsigned long long contextId() {
@@ -143,39 +172,29 @@ unsigned long long contextId() {
     return fn && fn(nullptr, &id) == CUDA_SUCCESS ? id : 0;
 }
 
-// Scratch for one call: the kept block of the current device if it is large enough, else a new one.
+// Scratch for one call: the kept block of the current context if it is large enough, else a new one.
 class ScratchLease {
 public:
     explicit ScratchLease(size_t bytes, cudaStream_t stream) {
         // A stream in capture takes none: what is captured would use it later.
         cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
         const bool plain = cudaStreamIsCapturing(stream, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone;
-        if (plain && cudaGetDevice(&device) == cudaSuccess && device >= 0 && device < kMaxDevices && (block.context = contextId())) {
-            KeptScratch kept{};
-            {
-                std::lock_guard<std::mutex> lock(g_keptMutex);
-                std::swap(kept, g_kept[device]);
+        if (plain && (block.context = contextId())) {
+            const KeptScratch kept = takeKept(block.context);
+            if (kept.base && kept.bytes >= bytes) {
+                block = kept;
+                return;
             }
-            if (kept.base && kept.context == block.context) {
-                if (kept.bytes >= bytes) {
-                    block = kept;
-                    return;
-                }
+            if (kept.base)
                 cudaFree(kept.base);
-            }
         }
         if (cudaMalloc(&block.base, bytes) != cudaSuccess)
             block.base = nullptr;
         block.bytes = bytes;
     }
     ~ScratchLease() {
-        if (block.base && block.context && block.bytes <= kKeptBytes && idle) {
-            std::lock_guard<std::mutex> lock(g_keptMutex);
-            if (!g_kept[device].base) {
-                g_kept[device] = block;
-                return;
-            }
-        }
+        if (block.base && block.context && block.bytes <= kKeptBytes && idle && putKept(block))
+            return;
         if (block.base)
             cudaFree(block.base);
     }
@@ -185,22 +204,15 @@ public:
     bool idle = false; // the stream has been waited for: the block may be kept
 
 private:
-    int device = 0;
     KeptScratch block{};
 };
 
 } // namespace
 
 void releaseSortScratch() {
-    int device = 0;
-    if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= kMaxDevices)
-        return;
-    KeptScratch kept{};
-    {
-        std::lock_guard<std::mutex> lock(g_keptMutex);
-        std::swap(kept, g_kept[device]);
-    }
-    if (kept.base && kept.context == contextId())
+    const unsigned long long context = contextId();
+    const KeptScratch kept = context ? takeKept(context) : KeptScratch{};
+    if (kept.base)
         cudaFree(kept.base);
 }
 

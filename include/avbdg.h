@@ -409,8 +409,8 @@ int avbdg_server_reset_stats(avbdg_server *server);
  * (src/radixsort.hpp:24-83, src/avbd/solver_broadphase.cpp:136-137). Keys must be below
  * 2^key_bits (1..64). On return d_keys[0 .. *unique_count) holds the distinct keys in order.
  * Runs on `stream` (a cudaStream_t; NULL = the default stream) and waits for it. Scratch is
- * allocated with cudaMalloc; up to 64 MiB of it, one block a device, is kept for the next call and
- * given back when a world, batch or server is destroyed or cannot allocate. */
+ * allocated with cudaMalloc; up to 64 MiB of it, one block a context, is kept for the context's next
+ * call and given back when a world, batch or server of the context is destroyed or cannot allocate. */
 int avbdg_sort_unique_keys(uint64_t *d_keys, int count, int key_bits, int *unique_count, void *stream);
 
 /* The same sort + unique for callers that cannot allocate device memory: a host that gives its

@@ -97,3 +97,20 @@ assert steps() == first
 def test_world_after_a_device_reset():
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     subprocess.run([sys.executable, "-c", RESET], cwd=root, check=True, timeout=120)
+
+
+# Sorts in two contexts in turn: each context's block stays its own and is found again.
+def test_sort_in_two_contexts(pkg, gpu, contexts):
+    fn, rng = sorter(pkg), np.random.default_rng(2)
+    free = []
+    for turn in range(5):
+        for where in (contextlib.nullcontext, contexts.other):
+            with where():
+                keys = rng.integers(0, 1 << 40, 1_000_000, dtype=np.uint64)
+                p, count = contexts.upload(keys), ctypes.c_int()
+                assert fn(p.value, keys.size, 40, ctypes.byref(count), None) == 0
+                out = np.empty_like(keys)
+                contexts.download(p, out)
+                assert np.array_equal(out[: count.value], np.unique(keys))
+        free.append(contexts.free_bytes())
+    assert free[1] == free[4]
