@@ -859,6 +859,16 @@ StepParams Engine::stepParams(real collisionDt) const {
 
 bool Engine::needGreedy() const { return nForces > 0 || !P.contact_only_overflow; }
 
+// A body count rounded up to the class of counts that one plan serves: eight to an octave, multiples of 8 at
+// least. The kernels read the count itself on the device; the launches take from the class their cluster sizes
+// (limits at 16, 24 and 64 bodies a CTA of 1 to 16, none inside a class) and their shared memory.
+static int sizeClass(int n) {
+    int g = 8;
+    while (16 * g <= n)
+        g *= 2;
+    return (n + g - 1) / g * g;
+}
+
 // Solver::broadPhase (solver_broadphase.cpp:85-186).
 // Host decisions of one step (everything the enqueued work depends on besides device counts).
 Engine::StepPlan Engine::planStep(int mode, int substeps, int rounds) {
@@ -907,14 +917,14 @@ Engine::StepPlan Engine::planStep(int mode, int substeps, int rounds) {
         const double density = ctrFresh && nBodies > 0 ? static_cast<double>(hostCtr[C_LIVE]) / nBodies : 2.5;
         if (worldsTake(count, bodies, density, nBodies > 0 ? static_cast<double>(nForces) / nBodies : 0.0)) {
             plan.worldCount = count;
-            plan.worldBodies = bodies;
+            plan.worldBodies = sizeClass(most);
         }
     }
     if (plan.greedy && worldAllowed && most <= colourWorldMost())
         for (plan.colourMost = 64; plan.colourMost < most;)
             plan.colourMost *= 2;
     if (worldAllowed && worlds() == 1 && plan.anyTree && most <= worldPairsMost())
-        plan.front = most;
+        plan.front = sizeClass(most);
     return plan;
 }
 
@@ -1087,7 +1097,16 @@ int Engine::enqueuePlan(const StepPlan &plan) {
         auto it = graphs.find(k);
         // A plan runs eagerly the first time it is seen after the cache was dropped and is
         // captured when it comes back, so plans that never recur cost no capture. Body and world
-        // counts are read on the device, so adding or removing worlds keeps the cache.
+        // counts are read on the device and only their classes are in the key, so adding or removing
+        // bodies and worlds keeps the cache while the classes stay.
+        if (it == graphs.end() && planSeen.size() >= kMostPlans) {
+            if (cudaStreamSynchronize(stream) != cudaSuccess) // the last graph may still run
+                return cudaCheck("step");
+            const bool seen = planSeen.count(k) != 0;
+            dropGraphs();
+            if (seen)
+                planSeen[k] = 1;
+        }
         const bool capture = it == graphs.end() && planSeen[k]++ > 0;
         if (it == graphs.end() && !capture) {
             if (!enqueueStep(plan))
@@ -1124,7 +1143,7 @@ int Engine::enqueuePlan(const StepPlan &plan) {
                     cudaEventDestroy(s.b);
                 }
                 spans.clear();
-                    if (!enqueueStep(plan))
+                if (!enqueueStep(plan))
                     return launchFailure();
             } else {
                 Graph gr{exec, launchCount() - before, {}};

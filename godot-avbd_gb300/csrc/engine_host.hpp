@@ -234,10 +234,10 @@ private:
         bool adjAtStart = false, anyTree = false, rebuild = false, forces = false, greedy = false;
         bool multiWorld = false, round = false;
         bool brute = false; // pairs by the all-pairs test within each world instead of the tree
-        // The step's second half as one launch, a cluster per world: worlds and the largest one's
-        // bodies, each rounded up to a power of two (0: separate launches).
+        // The step's second half as one launch, a cluster per world: worlds, rounded up to a power of two, and
+        // the largest one's bodies, rounded up to their class (sizeClass; 0: separate launches).
         int worldCount = 0, worldBodies = 0;
-        int front = 0; // the step's first half as two launches of one cluster: the world's bodies (0: separate)
+        int front = 0; // the step's first half as two launches of one cluster: the world's bodies, likewise (0: separate)
         int colourMost = 0; // colouring by a block a world, of up to this many bodies (0: across the store)
         bool worldMajor = false; // the compaction leaves the live manifolds in world order
         std::string key() const;
@@ -250,6 +250,7 @@ private:
     const std::vector<Span> *graphSpans = nullptr; // spans of the graph the last step ran
     std::map<std::string, Graph> graphs;
     std::map<std::string, int> planSeen; // plans run since the cache was dropped (capture on reuse)
+    static constexpr size_t kMostPlans = 128; // then the cache is dropped and begins anew
     bool useGraphs = true, capturing = false, lastGraph = false;
     std::string graphError;
     StepPlan planStep(int mode, int substeps, int rounds);
