@@ -964,9 +964,11 @@ void Engine::recordPhase(cudaEvent_t e) {
 }
 
 int Engine::broadPhase(const StepParams &sp, const StepPlan &plan) {
-    if (plan.adjAtStart)
-        launchAdjacency(d, stream);
     startPhase(0);
+    if (plan.adjAtStart) {
+        launchAdjacency(d, stream);
+        startPhase(kNoPhase);
+    }
     if (plan.front) {
         if (plan.rebuild) { // the tree's codes and order are dumped on the reference's schedule
             launchAabb(d, sp, stream);
@@ -1235,7 +1237,9 @@ void Engine::runWorlds(const StepParams &sp, const StepPlan &plan) {
     run.project = P.position_projection != 0 && sp.projIters > 0;
     run.colours = needGreedy();
     run.multiWorld = plan.multiWorld;
-    startPhase(2);
+    run.stampSolve = plan.mode == 0; // an interleaved step's brakes are its substeps'
+    if (!run.stampSolve)
+        startPhase(2);
     launchWorlds(d, sp, run, plan.worldCount, plan.worldBodies, stream);
     startPhase(kNoPhase);
 }

@@ -202,8 +202,16 @@ __device__ __forceinline__ unsigned long long nowNs() {
 // The start of a phase of the step, by its first kernel (an event between two kernels of a captured step
 // keeps them 8 us apart).
 __device__ __forceinline__ void stampPhase(const Dev &d) {
-    if (d.stamp > 0 && blockIdx.x == 0 && threadIdx.x == 0)
-        reinterpret_cast<unsigned long long *>(d.ctr + C_CLOCK)[d.stamp - 1] = nowNs();
+    if (d.stamp > 0 && blockIdx.x == 0 && threadIdx.x == 0) {
+        unsigned long long *clock = reinterpret_cast<unsigned long long *>(d.ctr + C_CLOCK);
+        clock[d.stamp - 1] = nowNs();
+        if (d.stamp == 2)
+            clock[2] = ~0ull; // (for stampSolve)
+    }
+}
+// The start of the solve in a launch that runs other phases too, by one thread of each world: the first's.
+__device__ __forceinline__ void stampSolve(const Dev &d) {
+    atomicMin(reinterpret_cast<unsigned long long *>(d.ctr + C_CLOCK) + 2, nowNs());
 }
 // List position of body g: the world's bodies in list order (reverse creation) occupy
 // [wBase, wBase + wCount).

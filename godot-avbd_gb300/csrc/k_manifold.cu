@@ -99,6 +99,7 @@ __global__ void adjInfoKernel(Dev d) {
 __global__ void adjClearKernel(Dev d) {
     pdlWait();
     pdlTrigger();
+    stampPhase(d);
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i <= d.NB)
         d.adjStart[i] = 0;

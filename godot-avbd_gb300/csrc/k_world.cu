@@ -1920,6 +1920,8 @@ __global__ void __launch_bounds__(kMaxWorldThreads, 1)
                 brakePhase(d, w, smem, r.substeps > 1 && !finished ? r.dt * static_cast<real>(r.substeps - step) : p.collisionDt);
             if (finished)
                 break;
+            if (r.stampSolve && w.rank == 0 && threadIdx.x == 0)
+                stampSolve(d);
             for (int i = threadIdx.x; i < w.nb; i += blockDim.x) {
                 const int g = w.b0 + i;
                 warmstartAt(d, p, g);
@@ -2035,6 +2037,8 @@ __global__ void __launch_bounds__(kWideThreads)
             }
             if (finished)
                 break;
+            if (r.stampSolve && tid == 0)
+                stampSolve(d);
             for (int g = base + tid; g < end; g += threads)
                 warmstartAt(d, p, g);
             clusterSync(size);

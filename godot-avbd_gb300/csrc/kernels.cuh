@@ -100,6 +100,7 @@ struct WorldRun {
     real dt;            // of a substep (the brake's window counts them down)
     real tolerance;     // projection: a pass whose deepest patch is within it is the last
     bool brake, project, colours, multiWorld;
+    bool stampSolve;    // the solve begins behind the first brake (else with the launch)
     unsigned rowBytes, smemBytes; // set by the launch
 };
 int worldTeamMax();

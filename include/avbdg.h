@@ -108,7 +108,11 @@ typedef struct avbdg_stats {
     int overflow_bodies;          /* overflowBodies */
     int update_bodies;            /* bodies in the update set */
     int steps;                    /* steps taken since creation */
-    /* last step, milliseconds: broad, graph (warm start + colouring + brake), solve, finish */
+    /* last step, milliseconds by the device's clock, from the start of its first kernel to the end of
+     * its last (what the host does before and after is not in it): broad (with the adjacency, where
+     * bodies or forces changed), graph (warm start + colouring + brake; an interleaved step's brakes
+     * are in its solve), solve, finish. Worlds stepped from the brake to the rebase in one launch have
+     * their finish in solve_ms, and finish_ms is 0. */
     double broad_ms, graph_ms, solve_ms, finish_ms, total_ms;
     int manifold_sides;           /* (manifold, side) pairs whose body moves: stamps per round */
     int graph_step;               /* 1 if the last step ran as one CUDA graph launch */

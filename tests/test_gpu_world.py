@@ -307,3 +307,39 @@ def test_dense_world_with_substeps(pkg, gpu, oracle, monkeypatch, params, forces
     assert same(here, run_forces(gpu, capi, world, params, steps=6, interleaved=(3, 2)))
     if not forces:
         assert same(here, run_forces(oracle, capi, world, params, steps=6, interleaved=(3, 2)))
+
+
+# A step's phases by either route: the brake counts with the warm start ("graph"), a chain of 300 candidates here, and the
+# adjacency that a new force makes a step rebuild first counts with the broad phase.
+@pytest.mark.parametrize("separate", ["0", "1"])
+def test_brake_and_adjacency_phases(pkg, gpu, monkeypatch, separate):
+    from test_gpu_waits import approaching_column
+
+    monkeypatch.setenv("AVBDG_NO_WORLD", separate)
+    capi = pkg.capi
+
+    def least(margin):
+        p = gpu.default_params()
+        p.speculative_margin = margin
+        w = capi.World(gpu, p, max_bodies=301)
+        w.add_bodies(approaching_column(pkg, 300))
+        begin = w.state()
+        begin[2][:] = [0, 0, 0]
+        times = []
+        for _ in range(12):
+            w.set_state(*begin)
+            w.step()
+            times.append(w.stats().graph_ms)
+        return min(times)
+
+    assert least(0.05) - least(0.0) > 0.05
+    w = pkg.scenes.instantiate(gpu, pkg.scenes.lattice(nx=40, ny=40, nz=16))
+    w.step(3)
+    fresh, plain = [], []
+    for k in range(8):
+        w.add_ignore_collision(1 + 2 * k, 2 + 2 * k)
+        w.step()
+        fresh.append(w.stats().broad_ms)
+        w.step()
+        plain.append(w.stats().broad_ms)
+    assert np.median(fresh) - np.median(plain) > 0.008  # its seven launches take 2 us each at least
