@@ -912,7 +912,9 @@ Engine::StepPlan Engine::planStep(int mode, int substeps, int rounds) {
             sortLiveByWorld();
         liveByWorld = plan.worldMajor || worlds() <= 1; // (a single world's order is its own)
     }
-    if (worldAllowed && (plan.worldMajor || worlds() == 1)) {
+    // A profiled step runs the separate launches, whose times are asked for (the state is the same).
+    const bool fused = worldAllowed && !profiling;
+    if (fused && (plan.worldMajor || worlds() == 1)) {
         // Manifolds a body in the last checked step (a store's first step: a settled pile's).
         const double density = ctrFresh && nBodies > 0 ? static_cast<double>(hostCtr[C_LIVE]) / nBodies : 2.5;
         if (worldsTake(count, bodies, density, nBodies > 0 ? static_cast<double>(nForces) / nBodies : 0.0)) {
@@ -923,7 +925,7 @@ Engine::StepPlan Engine::planStep(int mode, int substeps, int rounds) {
     if (plan.greedy && worldAllowed && most <= colourWorldMost())
         for (plan.colourMost = 64; plan.colourMost < most;)
             plan.colourMost *= 2;
-    if (worldAllowed && worlds() == 1 && plan.anyTree && most <= worldPairsMost())
+    if (fused && worlds() == 1 && plan.anyTree && most <= worldPairsMost())
         plan.front = sizeClass(most);
     return plan;
 }

@@ -244,7 +244,8 @@ int avbdg_world_get_stats(avbdg_world *world, avbdg_stats *out);
 int avbdg_world_digest(avbdg_world *world, uint64_t *out);
 
 /* Device time of the hot kernels, accumulated over steps while profiling is on (CUDA events on
- * the world's stream around each launch). Diagnostics beside the reference's PhaseTimes
+ * the world's stream around each launch; a profiled step runs these kernels even where an ordinary
+ * one has a single launch for several of them, with the same result). Diagnostics beside the reference's PhaseTimes
  * (src/avbd/solver.h:251-275), which time the same phases on the CPU. */
 typedef struct avbdg_kernel_times {
     double manifold_ms;   /* dual + stamp pass over manifolds (one launch per round) */

@@ -343,3 +343,23 @@ def test_brake_and_adjacency_phases(pkg, gpu, monkeypatch, separate):
         w.step()
         plain.append(w.stats().broad_ms)
     assert np.median(fresh) - np.median(plain) > 0.008  # its seven launches take 2 us each at least
+
+
+# Profiled steps of a world that is otherwise stepped in one launch: each kernel timed, the state the same.
+def test_profiled_world(pkg, gpu, monkeypatch):
+    monkeypatch.setenv("AVBDG_NO_TUNE", "1")
+    capi = pkg.capi
+    worlds = [capi.World(gpu, gpu.default_params(), max_bodies=301) for _ in range(2)]
+    for w in worlds:
+        w.add_bodies(heap(capi, 300, 5))
+        w.step(4)
+    worlds[0].set_profiling(True)
+    for w in worlds:
+        w.step(6)
+    kt, rounds = worlds[0].take_kernel_times(), gpu.default_params().iterations
+    assert (kt.steps, kt.manifold_launches, kt.body_launches, kt.narrow_launches) == (6, 6 * rounds, 6 * rounds, 6)
+    assert min(kt.manifold_ms, kt.body_ms, kt.narrow_ms) > 0
+    worlds[0].set_profiling(False)
+    for w in worlds:
+        w.step(4)
+    assert same([worlds[0].state()], [worlds[1].state()]) and worlds[0].stats().kernel_launches == worlds[1].stats().kernel_launches
