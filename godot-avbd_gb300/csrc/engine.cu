@@ -1090,6 +1090,8 @@ void Engine::dropGraphs() {
 // plans, whose graphs carry the span events, are cached apart), or eagerly the first time, when
 // graphs are disabled, during a tuning trial or when a capture failed.
 int Engine::enqueuePlan(const StepPlan &plan) {
+    if (const int ring = needRing()) // nothing is enqueued whose counters could not come back
+        return ring;
     launchBase = launchCount();
     graphSpans = nullptr;
     lastGraph = false;
@@ -1309,9 +1311,6 @@ int Engine::needRing() {
 
 int Engine::finishStep() {
     launches = launchCount() - launchBase;
-    const int ring = needRing();
-    if (ring)
-        return ring;
     launchPublish(d, ctrRing, stream);
     if (cudaStreamSynchronize(stream) != cudaSuccess)
         return cudaCheck("step");
@@ -1429,8 +1428,6 @@ int Engine::stepMany(int count, int substeps, int rounds) {
         const int r = rounds > 0 ? std::max(1, rounds) : std::max(2, (P.iterations + substeps - 1) / substeps);
         return planStep(1, substeps, r);
     };
-    if (const int ring = needRing())
-        return ring;
     int queued = -1; // ring slot of the step whose counters are not checked yet
     for (int i = 0; i < count; i++) {
         if (profiling || tuning) {
