@@ -30,3 +30,23 @@ def test_mass_range(pkg, gpu, oracle, density):
     for a, b in zip(*states):
         for x, y in zip(a, b):
             assert np.array_equal(x, y, equal_nan=True)
+
+
+def test_equal_to_division(pkg, tmp_path):
+    """`quotient` itself beside the compiler's division, compiled with the library's flags: 16 million pairs over its
+    range, with all-ones and short mantissas and at the range's ends, zeros of both signs; and that it refuses what
+    is outside its range and nothing inside it."""
+    import ctypes
+    import os
+    import subprocess
+
+    from avbd_gb300 import build
+
+    here = os.path.dirname(os.path.abspath(__file__))
+    lib = str(tmp_path / "quotients.so")
+    subprocess.run([build.nvcc()] + build.NVCC_FLAGS + ["-I" + build.CSRC, "-shared", os.path.join(here, "cuda", "quotients.cu"), "-o", lib],
+                   check=True)
+    out = (ctypes.c_ulonglong * 4)()
+    assert ctypes.CDLL(lib).check_quotients(out) == 0
+    wrong, refused, taken_outside, taken = out
+    assert (wrong, refused, taken_outside) == (0, 0, 0) and taken > 10_000_000
