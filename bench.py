@@ -36,6 +36,7 @@ Multi-GPU: one independent replica per rank (the path does not shard a single sc
 """
 
 import argparse
+import contextlib
 import ctypes
 import json
 import os
@@ -186,6 +187,17 @@ def traffic_per_launch(workload, algorithmic_bytes):
     return None if ratio is None else ratio * algorithmic_bytes
 
 
+@contextlib.contextmanager
+def step_events():
+    """Worlds and batches made here report the device time of a step between two CUDA events on the
+    library's stream, around the step's launches (AVBDG_STEP_EVENTS)."""
+    os.environ["AVBDG_STEP_EVENTS"] = "1"
+    try:
+        yield
+    finally:
+        del os.environ["AVBDG_STEP_EVENTS"]
+
+
 def profiled_pass(w, flush, steps):
     """Per-launch kernel times for the rooflines: `steps` more steps of `w` (a world or a batch) with
     the library's profiling spans on (CUDA events around each timed kernel, on the library's stream),
@@ -300,7 +312,8 @@ def run_gpu(args, rank, world_size):
     os.environ.setdefault("CUDA_VISIBLE_DEVICES", str(local))
     sc, desc = workload(args.workload)
     gpu = pkg.gpu_api()
-    w = scenes.instantiate(gpu, sc)
+    with step_events():
+        w = scenes.instantiate(gpu, sc)
     dyn_mask = sc.density > 0
     flush = torch.empty(L2_FLUSH_BYTES // 4, dtype=torch.float32, device="cuda")
 
@@ -311,8 +324,8 @@ def run_gpu(args, rank, world_size):
     torch.cuda.synchronize()
 
     # The timed steps run without per-kernel profiling spans: their events would split the step's
-    # chain of dependent launches. Each step's device time comes from the events the library records
-    # at the step's phase boundaries on its own stream.
+    # chain of dependent launches. Each step's device time comes from the two events the library records
+    # around the step's launches on its own stream.
     step_ms = []
     sum_bytes = 0
     launches = 0
@@ -490,14 +503,15 @@ def run_batch(args, rank, world_size):
             b.add_scene(w)
         return b
 
-    batch = make_batch()
+    with step_events():
+        batch = make_batch()
     dynamic = sum(w.dynamic for w in worlds)
     flush = torch.empty(L2_FLUSH_BYTES // 4, dtype=torch.float32, device="cuda")
     batch.step(args.warmup)
     if world_size > 1:
         torch.distributed.barrier()
     torch.cuda.synchronize()
-    # Timed without per-kernel profiling spans (see run_gpu); the step's phase events give its time.
+    # Timed without per-kernel profiling spans (see run_gpu), by the events around each step.
     step_ms = []
     sum_bytes = 0
     launches = 0
@@ -550,7 +564,7 @@ def run_batch(args, rank, world_size):
     e2e = {"value": dynamic * e2e_steps * world_size / e2e_s, "unit": UNIT, "h2d_bytes_per_step": nbytes,
            "d2h_bytes_per_step": nbytes}
     # Where an end-to-end step goes, from a few more steps after the timed ones (each part timed
-    # alone on the host clock, the step's device time from its own events).
+    # alone on the host clock, the step's device time from its kernels' own clock).
     split = {"upload_ms": 0.0, "step_wall_ms": 0.0, "step_device_ms": 0.0, "download_ms": 0.0}
     split_steps = 5
     for _ in range(split_steps):

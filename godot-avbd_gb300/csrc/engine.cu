@@ -250,6 +250,11 @@ Engine::Engine(const avbdg_params &params, int maxBodies, int maxForces, int max
         tuned = tunedBase;
     }
     cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking);
+    const char *events = std::getenv("AVBDG_STEP_EVENTS");
+    stepEvents = events && events[0] == '1';
+    if (stepEvents)
+        for (cudaEvent_t &e : evStep)
+            cudaEventCreate(&e);
     armStore = P.jacobian_rebuild_distance > 0.0f;
     const int nb = std::max(maxBodies, 64);
     allocate(nb, std::max(1024, 8 * nb), std::max(maxForces, 16), std::max(4096, 16 * nb), std::max(maxWorlds, 1));
@@ -270,6 +275,9 @@ Engine::~Engine() {
             cudaEventDestroy(e);
     for (cudaEvent_t e : evPool)
         cudaEventDestroy(e);
+    for (cudaEvent_t e : evStep)
+        if (e)
+            cudaEventDestroy(e);
     if (stream)
         cudaStreamDestroy(stream);
 }
@@ -1098,6 +1106,12 @@ int Engine::enqueuePlan(const StepPlan &plan) {
     const bool trial = tuning && tuneTrial >= 0;
     if (trial)
         configureTrial();
+    // With stepEvents the step's device time starts when its work is handed to the stream: after a capture and
+    // instantiation (host work the device only waits for), before an eager enqueue or a launch.
+    const auto startClock = [&] {
+        if (stepEvents)
+            cudaEventRecord(evStep[0], stream);
+    };
     if (useGraphs && !trial) {
         const std::string k = plan.key() + (profiling ? "/profiled" : "");
         auto it = graphs.find(k);
@@ -1115,6 +1129,7 @@ int Engine::enqueuePlan(const StepPlan &plan) {
         }
         const bool capture = it == graphs.end() && planSeen[k]++ > 0;
         if (it == graphs.end() && !capture) {
+            startClock();
             if (!enqueueStep(plan))
                 return launchFailure();
         } else if (it == graphs.end()) {
@@ -1149,6 +1164,7 @@ int Engine::enqueuePlan(const StepPlan &plan) {
                     cudaEventDestroy(s.b);
                 }
                 spans.clear();
+                startClock();
                 if (!enqueueStep(plan))
                     return launchFailure();
             } else {
@@ -1158,15 +1174,19 @@ int Engine::enqueuePlan(const StepPlan &plan) {
             }
         }
         if (it != graphs.end()) {
+            startClock();
             cudaGraphLaunch(it->second.exec, stream);
             launchBase = launchCount() - it->second.launches; // kernels inside the graph
             graphSpans = &it->second.spans;
             lastGraph = true;
         }
     } else {
+        startClock();
         if (!enqueueStep(plan))
             return launchFailure();
     }
+    if (stepEvents)
+        cudaEventRecord(evStep[1], stream);
     timed = true;
     return AVBDG_OK;
 }
@@ -2047,6 +2067,9 @@ int Engine::stats(avbdg_stats &out) {
         out.solve_ms = t[2];
         out.finish_ms = t[3];
         out.total_ms = t[0] + t[1] + t[2] + t[3];
+        float ms = 0.0f;
+        if (stepEvents && cudaEventElapsedTime(&ms, evStep[0], evStep[1]) == cudaSuccess)
+            out.total_ms = ms;
     }
     return cudaCheck("stats");
 }

@@ -158,6 +158,8 @@ private:
     bool roomy() const;
     int colourSizes[kMaxColours + 1] = {};
     bool timed = false;
+    bool stepEvents = false; // AVBDG_STEP_EVENTS=1: total_ms between two events around the step
+    cudaEvent_t evStep[2] = {};
     std::string err;
     // Profiling: event pairs around the hot launches of the current step.
     bool profiling = false;

@@ -112,7 +112,9 @@ typedef struct avbdg_stats {
      * its last (what the host does before and after is not in it): broad (with the adjacency, where
      * bodies or forces changed), graph (warm start + colouring + brake; an interleaved step's brakes
      * are in its solve), solve, finish. Worlds stepped from the brake to the rebase in one launch have
-     * their finish in solve_ms, and finish_ms is 0. */
+     * their finish in solve_ms, and finish_ms is 0. With the environment variable AVBDG_STEP_EVENTS=1
+     * when the world is created, total_ms is the time between two CUDA events on its stream, around the
+     * step's launches. */
     double broad_ms, graph_ms, solve_ms, finish_ms, total_ms;
     int manifold_sides;           /* (manifold, side) pairs whose body moves: stamps per round */
     int graph_step;               /* 1 if the last step ran as one CUDA graph launch */

@@ -363,3 +363,21 @@ def test_profiled_world(pkg, gpu, monkeypatch):
     for w in worlds:
         w.step(4)
     assert same([worlds[0].state()], [worlds[1].state()]) and worlds[0].stats().kernel_launches == worlds[1].stats().kernel_launches
+
+
+# A step timed by two events around its launches: no less than its kernels' own clock shows, no more than the host waited.
+@pytest.mark.parametrize("graphs", ["0", "1"])
+def test_step_events(pkg, gpu, monkeypatch, graphs):
+    import time
+
+    monkeypatch.setenv("AVBDG_STEP_EVENTS", "1")
+    monkeypatch.setenv("AVBDG_NO_GRAPHS", graphs)
+    capi = pkg.capi
+    w = capi.World(gpu, gpu.default_params(), max_bodies=301)
+    w.add_bodies(heap(capi, 300, 5))
+    for _ in range(12):
+        begin = time.perf_counter()
+        w.step()
+        wall = 1000 * (time.perf_counter() - begin)
+        st = w.stats()
+        assert 0.95 * (st.broad_ms + st.graph_ms + st.solve_ms + st.finish_ms) < st.total_ms < wall
