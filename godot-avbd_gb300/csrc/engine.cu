@@ -1563,11 +1563,11 @@ public:
             return;
         }
         cudaGetLastError(); // (of a block that could not grow)
+        pageable.resize(hostBytes); // (may throw: before what the destructor would free)
         if (cudaMalloc(&own, devBytes) != cudaSuccess) {
             own = nullptr;
             return;
         }
-        pageable.resize(hostBytes);
         dev = static_cast<char *>(own);
         host = pageable.data();
     }
