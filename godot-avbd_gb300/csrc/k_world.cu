@@ -2173,6 +2173,13 @@ size_t worldRows(int threads) { return sizeof(real) * static_cast<size_t>(thread
 //                 387 / 509 (all 128 bodies a CTA); 9 of 1000-2048 (256 a CTA, too many for one) 685 / 586
 // So worlds of up to 72 bodies a CTA, or 128 where four CTAs and more share a world, in up to three waves of
 // CTAs, and a single world while it fits.
+// The fit is an estimate, from the store's mean density and without the terms of bodies that are coloured though no
+// force touches them (contact_only_overflow 0), and the host is not told which worlds did not fit. It need not be:
+// worldWideKernel, to which they are left, took no longer than the separate launches in any store tried:
+//   uneven worlds 300 bodies within one another and 1200 apart 902 / 1050, 16 worlds of 500 with 120 so 542 / 591
+//   all coloured  900 bodies 1025 / 2612, 1100: 1526 / 2601, 2000: 2690 / 3024, 8 worlds of 900 1344 / 3212, 4 of 1900
+//                 3100 / 3322
+//   with forces   150 bodies within one another, 12 forces 1074 / 3181, 100 forces 2153 / 3404
 bool worldsTake(int worlds, int bodies, double density, double forces) {
     const int team = worldTeam(worlds, bodies), per = divUp(bodies, team);
     if (worlds * team > 3 * smCount() || (worlds > 1 && per > (team >= 4 ? 128 : 72)))

@@ -20,8 +20,8 @@ constexpr int kSmallThreads = 1024;
 constexpr int kSmallItems = 16;
 constexpr int kSmallScanCap = kSmallThreads * kSmallItems;
 // Larger ones, up to kClusterScanCap, by one cluster: its CTAs hold up to 131,072 values at a time and tell
-// one another their sums. Microseconds here and by the other forms: 16,384 values 3.3 / 7.4 (one block), 30,000
-// 3.4 / 7.0 (three launches), 65,537 4.5 / 7.2; 452,000, in four turns, 23.3 / 12.8.
+// one another their sums. Microseconds here and by the other forms: 16,384 values 3.5 / 7.4 (one block), 30,000
+// 3.8 / 7.0 (three launches), 65,537 5.0 / 7.2; 452,000, in four turns, 23.3 / 12.8.
 constexpr int kBlockScanCap = 4096;
 constexpr int kClusterScanCap = 1 << 17;
 constexpr int kClusterItems = 8;

@@ -219,7 +219,9 @@ int avbdg_world_get_sleeping(avbdg_world *world, int first, int count, uint8_t *
 /* Solver::pick (src/avbd/solver_query.cpp:24-152) for `count` rays at once: ray i starts at
  * origins[3i..] along dirs[3i..] (not normalised; distances are in units of dir). out_body[i] is
  * the creation index of the nearest body hit whose layer meets `mask` (-1: none; the first in list
- * order wins a tie), out_local[3i..] the hit point in that body's frame. */
+ * order wins a tie), out_local[3i..] the hit point in that body's frame. Queries keep their scratch
+ * with the world, up to 16 MiB of device memory and 16 MiB pinned on the host, outside any device byte
+ * limit; a larger one, or one while another thread's runs, allocates its own for the call. */
 int avbdg_world_pick(avbdg_world *world, int count, const float *origins, const float *dirs, uint32_t mask,
                      int *out_body, float *out_local);
 /* Solver::collectAABB (src/avbd/solver_query.cpp:154-170): bodies whose tight bounds overlap
